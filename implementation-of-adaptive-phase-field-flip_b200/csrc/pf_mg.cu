@@ -1165,7 +1165,7 @@ __device__ void bt_local_vcycle(const BottomLevel* Ls, float* base, int l0, int 
     const int n = L.n0 * L.n1 * L.n2;
     for (int e = tid; e < n; e += NT) Pc[e] = AccT(0);
     __syncthreads();
-    const bool one_warp = n <= 256;
+    const bool one_warp = n <= 64;
     const AccT omc = (AccT)om;
     if (n <= 64 && (L.n2 & 1) == 0) {
       if (tid < 32) bt_coarsest_regs<AccT>(L, Pc, q.B, q.X, q.Y, q.Z, omc, coarsest, flux, tid);
@@ -1394,8 +1394,6 @@ __global__ void __launch_bounds__(BT_NT) k_bottom(const __grid_constant__ Bottom
 constexpr int BC_CTAS = 8;
 constexpr int BC_MAX_DIST = 4;
 constexpr int BC_NT = 512;  // threads per CTA (128 registers a thread)
-constexpr int kDenseMaxCells = 1024;  // largest level applied as a dense operator
-static_assert(kDenseMaxCells / BC_CTAS <= BC_NT, "dense rows of a CTA must fit its partial-sum buffer");
 
 template <class T, class TB> struct ClusterArgs {
   int nd;                           // distributed levels, [0] = top
@@ -1411,8 +1409,6 @@ template <class T, class TB> struct ClusterArgs {
   int flux;
   MGState* st;
   int want_mean, mixed;
-  const float* M;                   // dense operator of the levels below (null: CTA 0 runs them)
-  int nb;                           // its size: cells of the level below D[nd-1]
 };
 
 // floats of one CTA's slab of a distributed level: P, B (s planes), X (s+1
@@ -1596,16 +1592,6 @@ __global__ void __cluster_dims__(BC_CTAS, 1, 1) __launch_bounds__(BC_NT, 1) k_bo
   float* base = reinterpret_cast<float*>(bcsm);
   float* lbase = base;  // after the slabs (the layout is the same in every CTA)
   for (int l = 0; l < nd; ++l) lbase += bc_level_floats(a.D[l].n0, a.D[l].n1, a.D[l].n2);
-  auto align16 = [](float* p) {
-    return reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
-  };
-  // dense bottom: the full right-hand side of the level below, this CTA's rows
-  // of its solution and the partial sums of the product; otherwise CTA 0's
-  // levels and the coarsest solution
-  const bool dense = a.M != nullptr;
-  float* bfull = align16(lbase);
-  float* pd = align16(bfull + a.nb);
-  float* red = align16(pd + a.nb / BC_CTAS);
   AccT* Pc;
   {
     float* end = lbase;
@@ -1636,7 +1622,7 @@ __global__ void __cluster_dims__(BC_CTAS, 1, 1) __launch_bounds__(BC_NT, 1) k_bo
     if (a.b_scale) bt_load<TB, BC_NT>(L.B, src, cnt, *a.b_scale, tid);
     else bc_load(L.B, src, cnt, tid);
   }
-  if (rank == 0 && !dense) {
+  if (rank == 0) {
     for (int l = 0; l < nl; ++l) {
       const BottomLevel& G = a.L[l];
       const BtPtrs q = bt_ptrs(a.L, lbase, l);
@@ -1665,12 +1651,11 @@ __global__ void __cluster_dims__(BC_CTAS, 1, 1) __launch_bounds__(BC_NT, 1) k_bo
         cl.sync();
       }
     L.use_slot(cur[l]);
-    // coarse planes rank*s/2 .. : into the next slab, or into CTA 0's first
-    // level, or (dense) into every CTA's copy of the full right-hand side
+    // coarse planes rank*s/2 .. : into the next slab, or into CTA 0's first level
     const int C1 = L.n1 >> 1, C2 = L.n2 >> 1, hs = L.s >> 1, nc = hs * C1 * C2;
     const bool last = l + 1 == nd;
     float* Bc = !last ? bc_level(a.D, base, l + 1, rank, cl).B
-                      : dense ? bfull + (size_t)rank * nc : cl.map_shared_rank(bt_ptrs(a.L, lbase, 0).B, 0) + (size_t)rank * nc;
+                      : cl.map_shared_rank(bt_ptrs(a.L, lbase, 0).B, 0) + (size_t)rank * nc;
     const bool p2 = L.s1 >= 1 && L.s2 >= 1;
     for (int ec = tid; ec < nc; ec += BC_NT) {
       int I, J, K;
@@ -1692,42 +1677,16 @@ __global__ void __cluster_dims__(BC_CTAS, 1, 1) __launch_bounds__(BC_NT, 1) k_bo
         for (int bb = 0; bb < 2; ++bb)
 #pragma unroll
           for (int c2 = 0; c2 < 2; ++c2) acc += bc_residual(L, 2 * I + aa, 2 * J + bb, 2 * K + c2, a.flux);
-      const float v = roundT<T>(acc * a.rscale);
-      if (last && dense) {
-        for (int r = 0; r < BC_CTAS; ++r) cl.map_shared_rank(Bc, r)[ec] = v;
-      } else {
-        Bc[ec] = v;
-      }
+      Bc[ec] = roundT<T>(acc * a.rscale);
     }
     cl.sync();
   }
 
-  // ---- the levels below: the dense operator's rows of this CTA's coarse
-  // planes (partial sums over column chunks, added in chunk order), or CTA 0
-  if (dense) {
-    const int nb = a.nb, R = nb / BC_CTAS, row0 = rank * R;
-    const int ch = R >= BC_NT ? 1 : BC_NT / R;  // column chunks per row
-    const int cw = (nb + ch - 1) / ch;
-    for (int t = tid; t < R * ch; t += BC_NT) {
-      const int i = t % R, c = t / R;
-      const int m0 = c * cw, m1 = min(nb, m0 + cw);
-      float acc = 0.f;
-      for (int m = m0; m < m1; ++m) acc = fmaf(__ldg(a.M + (size_t)m * nb + row0 + i), bfull[m], acc);
-      red[t] = acc;
-    }
-    __syncthreads();
-    for (int i = tid; i < R; i += BC_NT) {
-      float v = 0.f;
-      for (int c = 0; c < ch; ++c) v += red[c * R + i];
-      pd[i] = v;
-    }
-    __syncthreads();
-  } else {
-    if (rank == 0)
-      bt_local_vcycle<T, AccT, BC_NT>(a.L, lbase, 0, nl, Pc, om, a.pre, a.post, a.coarsest, a.rscale, a.pscale,
-                                      a.flux, sred, &s_mean);
-    cl.sync();
-  }
+  // ---- the levels below, on CTA 0
+  if (rank == 0)
+    bt_local_vcycle<T, AccT, BC_NT>(a.L, lbase, 0, nl, Pc, om, a.pre, a.post, a.coarsest, a.rscale, a.pscale, a.flux,
+                                    sred, &s_mean);
+  cl.sync();
 
   // ---- up the distributed levels: prolongation, post-smoothing with the colours reversed
   for (int l = nd - 1; l >= 0; --l) {
@@ -1738,9 +1697,6 @@ __global__ void __cluster_dims__(BC_CTAS, 1, 1) __launch_bounds__(BC_NT, 1) k_bo
     if (l + 1 < nd) {
       Pcoarse = bc_level(a.D, base, l + 1, rank, cl).P;
       cplane0 = L.i0 >> 1;
-    } else if (dense) {
-      Pcoarse = pd;
-      cplane0 = rank * (L.s >> 1);
     } else {
       Pcoarse = cl.map_shared_rank(bt_ptrs(a.L, lbase, 0).P, 0);
       cplane0 = 0;
@@ -1802,15 +1758,16 @@ __global__ void __cluster_dims__(BC_CTAS, 1, 1) __launch_bounds__(BC_NT, 1) k_bo
   }
 }
 
-// ---- the dense bottom operator, one column per CTA: the V-cycle of the
-// levels below the cluster's slabs (bt_local_vcycle, DB_NT threads) applied to
-// the unit right-hand side e_m, written to M[m * nb + i]
+// ---- the dense operator of the cluster kernel's last levels, one column per
+// CTA: their V-cycle (bt_local_vcycle, DB_NT threads, nothing rounded to the
+// storage type) applied to the unit right-hand side e_m, written to
+// M[m * nb + i] in the type of the coarsest solve
 constexpr int DB_NT = 128;
 
 template <class T> struct DenseBuildArgs {
   int nl;
   BottomLevel L[PF_MG_MAX_LEVELS];
-  float* M;
+  void* M;
   float omega;
   int pre, post, coarsest;
   float rscale, pscale;
@@ -1843,12 +1800,17 @@ __global__ void __launch_bounds__(DB_NT) k_bottom_dense_build(const __grid_const
     }
   }
   __syncthreads();
-  bt_local_vcycle<T, AccT, DB_NT>(a.L, base, 0, a.nl, Pc, a.omega, a.pre, a.post, a.coarsest, a.rscale, a.pscale,
-                                  a.flux, sred, &s_mean);
+  bt_local_vcycle<float, AccT, DB_NT>(a.L, base, 0, a.nl, Pc, a.omega, a.pre, a.post, a.coarsest, a.rscale, a.pscale,
+                                      a.flux, sred, &s_mean);
   const float* P0 = bt_ptrs(a.L, base, 0).P;
   const int nb = a.L[0].n0 * a.L[0].n1 * a.L[0].n2;
-  for (int i = tid; i < nb; i += DB_NT) a.M[(size_t)m * nb + i] = P0[i];
+  AccT* M = reinterpret_cast<AccT*>(a.M) + (size_t)m * nb;
+  for (int i = tid; i < nb; i += DB_NT) M[i] = a.nl == 1 ? Pc[i] + (AccT)(-s_mean) : (AccT)P0[i];
 }
+
+}  // namespace pf
+#include "pf_mg_coarse.cuh"
+namespace pf {
 
 // --------------------------------------------------------------- CG vector kernels
 // Sum of b (for the mean); last CTA stores c_shift = float(-sum/n).
@@ -2204,8 +2166,11 @@ struct pf_mg_plan {
   bool bottom_stage;   // bottom_smem includes the 16-bit staging area
   int bc_nd;           // > 0: levels lb .. lb+bc_nd-1 run distributed on a CTA cluster (k_bottom_cluster)
   size_t bc_smem;      // dynamic shared memory per CTA of the cluster kernel
-  int dense_nb;        // > 0: the levels below the slabs run as a dense nb x nb operator in bottom_op
-  float* bottom_op;
+  bool coarse;         // levels lb .. run in k_coarse (args in cc), else in the kernels above
+  int cc_nq;           // quads per thread of its instantiation
+  size_t cc_smem;
+  pf::CcArgs cc;       // geometry; the pointers are set per launch
+  int dense_l0;        // first level of the dense operator (cc.nb > 0)
   cudaStream_t cap_stream;
   cudaGraphExec_t exec[2];
   size_t exec_nodes[2];
@@ -2463,8 +2428,6 @@ int launch_bottom_cluster(pf_mg_plan* P, const TB* b, const float* b_scale, bool
   a.st = ST(P);
   a.want_mean = want_mean ? 1 : 0;
   a.mixed = mixed(P) ? 1 : 0;
-  a.M = P->dense_nb ? P->bottom_op : nullptr;
-  a.nb = P->dense_nb;
   if (mixed(P)) k_bottom_cluster<T, TB, double><<<BC_CTAS, BC_NT, P->bc_smem, s>>>(a);
   else k_bottom_cluster<T, TB, float><<<BC_CTAS, BC_NT, P->bc_smem, s>>>(a);
   PF_LAUNCHED();
@@ -2472,8 +2435,63 @@ int launch_bottom_cluster(pf_mg_plan* P, const TB* b, const float* b_scale, bool
   return PF_OK;
 }
 
+template <class T> void* coarse_kernel(int nq) {
+  return nq <= 1 ? (void*)k_coarse<T, 1> : nq <= 2 ? (void*)k_coarse<T, 2> : (void*)k_coarse<T, 3>;
+}
+
+cudaLaunchConfig_t coarse_config(int C, size_t smem, cudaStream_t s, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(C);
+  cfg.blockDim = dim3(CC_NT);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cfg;
+}
+
+template <class T, class TB>
+int launch_coarse(pf_mg_plan* P, const TB* b, const float* b_scale, bool want_mean, cudaStream_t s, T** out) {
+  CcArgs a = P->cc;
+  LV<T> V0 = view<T>(P, P->lb);
+  for (int l = 0; l < a.nl; ++l) {
+    LV<T> V = view<T>(P, P->lb + l);
+    a.L[l].bx = V.bx;
+    a.L[l].by = V.by;
+    a.L[l].bz = V.bz;
+  }
+  a.M = P->d.bottom_op;
+  a.b = b;
+  a.b_f32 = std::is_same<TB, float>::value ? 1 : 0;
+  a.b_scale = b_scale;
+  a.p_out = V0.p0;
+  a.omega = P->d.omega;
+  a.pre = P->d.pre;
+  a.post = P->d.post;
+  a.coarsest = P->d.coarsest;
+  a.rscale = mixed(P) ? 0.125f : 1.f;
+  a.pscale = mixed(P) ? 2.f : 1.f;
+  a.flux = FLUX(P);
+  a.st = ST(P);
+  a.want_mean = want_mean ? 1 : 0;
+  a.mixed = mixed(P) ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  const cudaLaunchConfig_t cfg = coarse_config(a.C, P->cc_smem, s, attr);
+  void* args[] = {&a};
+  PF_CUDA_TRY(cudaLaunchKernelExC(&cfg, coarse_kernel<T>(P->cc_nq), args));
+  PF_LAUNCHED();
+  *out = V0.p0;
+  return PF_OK;
+}
+
 template <class T, class TB>
 int launch_bottom(pf_mg_plan* P, const TB* b, const float* b_scale, bool want_mean, cudaStream_t s, T** out) {
+  if (P->coarse) return launch_coarse<T, TB>(P, b, b_scale, want_mean, s, out);
   if (P->bc_nd > 0) return launch_bottom_cluster<T, TB>(P, b, b_scale, want_mean, s, out);
   BottomArgs<T, TB> a;
   const int lb = P->lb;
@@ -2752,17 +2770,17 @@ int solve_impl(pf_mg_plan* P, const float* b, float* x, float tol, int max_iter,
   return PF_OK;
 }
 
-// the dense operator of the levels below the cluster's slabs, one column per CTA
+// the dense operator of the cluster kernel's last levels, one column per CTA
 template <class T> int launch_dense_build(pf_mg_plan* P, cudaStream_t s) {
+  using Acc = typename CcAcc<T>::type;
   DenseBuildArgs<T> a;
-  const int l0 = P->lb + P->bc_nd;
-  a.nl = P->d.nlev - l0;
+  a.nl = P->d.nlev - P->dense_l0;
   size_t floats = 0;
   for (int l = 0; l < a.nl; ++l) {
-    a.L[l] = bottom_level<T>(P, l0 + l);
+    a.L[l] = bottom_level<T>(P, P->dense_l0 + l);
     floats += bottom_level_floats(a.L[l].n0, a.L[l].n1, a.L[l].n2);
   }
-  a.M = P->bottom_op;
+  a.M = P->d.bottom_op;
   a.omega = P->d.omega;
   a.pre = P->d.pre;
   a.post = P->d.post;
@@ -2772,8 +2790,7 @@ template <class T> int launch_dense_build(pf_mg_plan* P, cudaStream_t s) {
   a.flux = FLUX(P);
   const BottomLevel& Lc = a.L[a.nl - 1];
   const size_t smem = floats * sizeof(float) + 16 + (size_t)Lc.n0 * Lc.n1 * Lc.n2 * sizeof(double);
-  if (mixed(P)) k_bottom_dense_build<T, double><<<P->dense_nb, DB_NT, smem, s>>>(a);
-  else k_bottom_dense_build<T, float><<<P->dense_nb, DB_NT, smem, s>>>(a);
+  k_bottom_dense_build<T, Acc><<<P->cc.nb, DB_NT, smem, s>>>(a);
   PF_LAUNCHED();
   return PF_OK;
 }
@@ -2798,7 +2815,7 @@ template <class T> int build_impl(pf_mg_plan* P, cudaStream_t s) {
       PF_LAUNCHED();
     }
   }
-  if (P->dense_nb) {
+  if (P->coarse && P->cc.nb > 0) {
     const int rc = launch_dense_build<T>(P, s);
     if (rc != PF_OK) return rc;
   }
@@ -2820,6 +2837,8 @@ template <class T> int precondition_impl(pf_mg_plan* P, const float* r, float* z
   return PF_OK;
 }
 
+constexpr int kCcSmemMax = 224 * 1024;  // dynamic shared memory of a k_coarse CTA
+
 template <class T> cudaError_t set_smem_attrs() {
   const int mx = 220 * 1024, tile = (int)TileDims<4>::SMEM;
   cudaError_t e = cudaSuccess;
@@ -2834,8 +2853,12 @@ template <class T> cudaError_t set_smem_attrs() {
   chk(cudaFuncSetAttribute(k_bottom_cluster<T, T, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
   chk(cudaFuncSetAttribute(k_bottom_cluster<T, float, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
   chk(cudaFuncSetAttribute(k_bottom_cluster<T, T, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  chk(cudaFuncSetAttribute(k_bottom_dense_build<T, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
-  chk(cudaFuncSetAttribute(k_bottom_dense_build<T, double>, cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  chk(cudaFuncSetAttribute(k_bottom_dense_build<T, typename CcAcc<T>::type>,
+                           cudaFuncAttributeMaxDynamicSharedMemorySize, mx));
+  for (int nq : {1, 2, 3}) {
+    chk(cudaFuncSetAttribute(coarse_kernel<T>(nq), cudaFuncAttributeMaxDynamicSharedMemorySize, kCcSmemMax));
+    chk(cudaFuncSetAttribute(coarse_kernel<T>(nq), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  }
   chk(cudaFuncSetAttribute(k_rb_tile<T, float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
   chk(cudaFuncSetAttribute(k_rb_tile<T, T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
   chk(cudaFuncSetAttribute(k_rb_tile_tma<4, SW_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2867,11 +2890,120 @@ struct BottomSel {
   bool bottom_stage = false;
   int bc_nd = 0;           // cluster kernel: distributed levels
   size_t bc_smem = 0;
-  int dense_nb = 0;        // dense operator of the levels below the slabs: its size (cells)
-  size_t bc_smem_dense = 0;
 };
 
-// The bottom of a plan's V-cycle (pf_mg_plan_create, pf_mg_bottom_op_floats).
+// Geometry of k_coarse for the levels lv .. of a plan.  false where they do
+// not fit.  Every limit is one of capacity: a thread holds 2 quads of cells in
+// its registers (3, with a few spills, where a level fits no other way), a CTA
+// kCcSmemMax bytes.  A level of up to CC_NT * 2 quads stays on one CTA, where a
+// half-sweep needs no exchange.
+bool coarse_geometry(const pf_mg_desc* desc, int lv, CcArgs* a, int* nq, size_t* smem, int* dense_l0) {
+  std::memset(a, 0, sizeof(*a));
+  const int nlev = desc->nlev;
+  const bool mx = desc->precision != PF_PREC_FP32;
+  auto cells = [&](int l) { return (long long)desc->lev[l].nx * desc->lev[l].ny * desc->lev[l].nz; };
+  int ld = lv + 1;  // first level of the dense operator, never the top one
+  while (ld < nlev && cells(ld) > kCcDenseMax) ++ld;
+  *dense_l0 = ld;
+  a->nl = ld - lv;
+  constexpr long long kLocal = 2 * CC_NT, kMost = 3 * CC_NT;
+  int local = 0, dist = 0;
+  for (int l = 0; l < a->nl; ++l) {
+    const pf_mg_level& G = desc->lev[lv + l];
+    CcLevel& L = a->L[l];
+    L.n0 = G.nx;
+    L.n1 = G.ny;
+    L.n2 = G.nz;
+    if (G.nx > 8000 || (long long)G.ny * G.nz > 4 * kMost) return false;  // also the range of CcDiv
+    L.hk = 2 * ((G.nz + 3) / 4);
+    const long long quads = (long long)L.n0 * L.n1 * L.hk / 2;
+    if (quads <= kLocal) ++local;
+    else if (quads > kMost * CC_MAXC) return false;
+    else ++dist;
+  }
+  a->C = (dist > 0 || ld < nlev) ? CC_MAXC : 1;
+  // local levels on CTAs of their own at the end of the cluster, so that each
+  // keeps its coefficients in registers throughout; slabs on the others, or on
+  // all where they need the room
+  int next_local = a->C - 1;
+  long long most = 1;
+  for (int l = a->nl - 1; l >= 0; --l) {
+    CcLevel& L = a->L[l];
+    const long long plane = (long long)L.n1 * L.hk / 2;
+    if (L.n0 * plane <= kLocal) {
+      L.A = 1;
+      L.c0 = next_local > 0 ? next_local-- : 0;
+      L.smax = L.n0;
+    } else {
+      L.c0 = 0;
+      L.A = L.n0 < a->C - local ? L.n0 : a->C - local;
+      if (L.A < 2 || (L.n0 + L.A - 1) / L.A * plane > kLocal) L.A = L.n0 < a->C ? L.n0 : a->C;
+      L.smax = (L.n0 + L.A - 1) / L.A;
+      if (L.A < 2 || L.smax * plane > kMost) return false;
+    }
+    if (L.smax * plane > most) most = L.smax * plane;
+    for (int r = 0; r <= L.A; ++r) L.lo[r] = (short)(r * L.n0 / L.A);
+    L.by_qpl = CcDiv::of((int)plane);
+    L.by_hq = CcDiv::of(L.hk / 2);
+    L.by_n0 = CcDiv::of(L.n0);
+    L.by_ck = CcDiv::of(L.n2 > 1 ? L.n2 / 2 : 1);
+    L.by_crows = CcDiv::of(L.n1 > 1 && L.n2 > 1 ? (L.n1 / 2) * (L.n2 / 2) : 1);
+  }
+  *nq = (int)((most + CC_NT - 1) / CC_NT);
+  // shared memory: what starts at zero first (in 16-byte units)
+  size_t off = 0, scr = 0;
+  auto take = [&off](size_t floats) {
+    const size_t o = off;
+    off = (off + floats + 3) / 4 * 4;
+    return (int)o;
+  };
+  for (int l = 0; l < a->nl; ++l) {
+    CcLevel& L = a->L[l];
+    L.oP = take(2 * (size_t)(L.smax + 2) * L.n1 * L.hk);
+  }
+  const bool dense = ld < nlev;
+  if (!dense && mx && a->L[a->nl - 1].A == 1) {
+    const CcLevel& L = a->L[a->nl - 1];
+    a->oPd = take(4 * (size_t)(L.n0 + 2) * L.n1 * L.hk);
+  }
+  a->zero_floats = (int)off;
+  a->oBar = take(8);
+  for (int l = 0; l < a->nl; ++l) {
+    CcLevel& L = a->L[l];
+    if (l > 0) L.oB = take(2 * (size_t)L.smax * L.n1 * L.n2);
+    const size_t q = (size_t)L.smax * L.n1 * L.hk;
+    if (q > scr) scr = q;
+  }
+  a->oS = take(scr);
+  if (dense) {
+    const pf_mg_level& D = desc->lev[ld];
+    const size_t es = mx ? 2 : 1;  // floats per element of the operator
+    a->nb = (int)cells(ld);
+    a->bn1 = D.ny;
+    a->bn2 = D.nz;
+    a->cd = a->C - 1;
+    a->oDB = take(2 * (size_t)a->nb);
+    a->oDP = take(a->nb);
+    a->oDb = take(a->nb);
+    a->oDr = take(es * CC_NT);
+    const size_t rows = (size_t)((a->nb + a->C - 1) / a->C) * a->nb * es;
+    a->oDM = (off + rows) * sizeof(float) <= (size_t)kCcSmemMax ? take(rows) : -1;
+  }
+  *smem = off * sizeof(float);
+  return *smem <= (size_t)kCcSmemMax;
+}
+
+// the finest level from which k_coarse can run, -1 where there is none or
+// PFFLIP_MG_BOTTOM=cta / cluster asks for the kernels before it
+int select_coarse(const pf_mg_desc* desc, CcArgs* a, int* nq, size_t* smem, int* dense_l0) {
+  const char* env = std::getenv("PFFLIP_MG_BOTTOM");
+  if (env && (std::strcmp(env, "cta") == 0 || std::strcmp(env, "cluster") == 0)) return -1;
+  for (int lv = 0; lv < desc->nlev; ++lv)
+    if (coarse_geometry(desc, lv, a, nq, smem, dense_l0)) return lv;
+  return -1;
+}
+
+// The bottom of a plan's V-cycle without k_coarse: one CTA, or the 8-CTA cluster.
 BottomSel select_bottom(const pf_mg_desc* desc) {
   BottomSel r;
   // bottom kernel: the deepest run of levels that each fit kBottomMaxCells and
@@ -2908,7 +3040,6 @@ BottomSel select_bottom(const pf_mg_desc* desc) {
   {
     const char* env = std::getenv("PFFLIP_MG_BOTTOM");
     const bool allow = !(env && std::strcmp(env, "cta") == 0);
-    const bool allow_dense = !(env && (std::strcmp(env, "cta") == 0 || std::strcmp(env, "cluster") == 0));
     const int nlev = desc->nlev;
     const pf_mg_level& Lc = desc->lev[nlev - 1];
     for (int lv = 0; allow && lv < r.lb; ++lv) {
@@ -2933,16 +3064,6 @@ BottomSel select_bottom(const pf_mg_desc* desc) {
       r.bc_nd = nd;
       r.bc_smem = bytes;
       r.lb = lv;
-      // dense bottom: the levels below the slabs as one operator on the first of
-      // them, each CTA applying the rows of its own coarse planes
-      const pf_mg_level& F = desc->lev[lv + nd];
-      const int nb = F.nx * F.ny * F.nz;
-      if (allow_dense && nb <= kDenseMaxCells && F.nx % BC_CTAS == 0) {
-        size_t dfl = 0;
-        for (int l = lv; l < lv + nd; ++l) dfl += bc_level_floats(desc->lev[l].nx, desc->lev[l].ny, desc->lev[l].nz);
-        r.dense_nb = nb;
-        r.bc_smem_dense = (dfl + 4 + (size_t)nb + 4 + (size_t)(nb / BC_CTAS) + 4 + BC_NT) * sizeof(float);
-      }
       break;
     }
   }
@@ -3005,17 +3126,6 @@ int pf_mg_plan_create(const pf_mg_desc* desc, pf_mg_plan** out) {
   for (int lv = 0; lv < desc->nlev; ++lv) {
     P->lp_scale[lv] = std::ldexp(desc->coef_scale > 0.f ? desc->coef_scale : 1.f, -2 * lv);
   }
-  {
-    const BottomSel sel = select_bottom(desc);
-    P->lb = sel.lb;
-    P->bottom_smem = sel.bottom_smem;
-    P->bottom_stage = sel.bottom_stage;
-    P->bc_nd = sel.bc_nd;
-    P->bc_smem = sel.bc_smem;
-    P->dense_nb = (sel.dense_nb > 0 && desc->bottom_op) ? sel.dense_nb : 0;
-    if (P->dense_nb) P->bc_smem = sel.bc_smem_dense;
-    P->bottom_op = desc->bottom_op;
-  }
   cudaError_t e = cudaStreamCreateWithFlags(&P->cap_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaHostAlloc((void**)&P->h_state[0], sizeof(pf::MGState) * 2, cudaHostAllocDefault);
   if (e == cudaSuccess) {
@@ -3028,13 +3138,34 @@ int pf_mg_plan_create(const pf_mg_desc* desc, pf_mg_plan** out) {
     pf_mg_plan_destroy(P);
     return PF_ERR_CUDA;
   }
-  e = set_smem_attrs<float>();
-  if (e == cudaSuccess) e = set_smem_attrs<__half>();
-  if (e == cudaSuccess) e = set_smem_attrs<__nv_bfloat16>();
+  e = set_smem_attrs<float>();  // pf_mg_smooth runs in FP32 whatever the plan's storage
+  if (e == cudaSuccess && desc->precision == PF_PREC_FP16) e = set_smem_attrs<__half>();
+  if (e == cudaSuccess && desc->precision == PF_PREC_BF16) e = set_smem_attrs<__nv_bfloat16>();
   if (e != cudaSuccess) {
     pf::set_cuda_error(e, "cudaFuncSetAttribute (shared memory)");
     pf_mg_plan_destroy(P);
     return PF_ERR_CUDA;
+  }
+  // k_coarse where its cluster can be resident; the dense operator needs its buffer
+  P->lb = select_coarse(desc, &P->cc, &P->cc_nq, &P->cc_smem, &P->dense_l0);
+  P->coarse = P->lb >= 0 && (P->cc.nb == 0 || (desc->bottom_op && (reinterpret_cast<uintptr_t>(desc->bottom_op) & 7u) == 0));
+  if (P->coarse && P->cc.C > 8) {
+    cudaLaunchAttribute attr[2];
+    const cudaLaunchConfig_t cfg = coarse_config(P->cc.C, P->cc_smem, nullptr, attr);
+    void* k = desc->precision == PF_PREC_FP16   ? coarse_kernel<__half>(P->cc_nq)
+              : desc->precision == PF_PREC_BF16 ? coarse_kernel<__nv_bfloat16>(P->cc_nq)
+                                                : coarse_kernel<float>(P->cc_nq);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) P->coarse = false;
+    cudaGetLastError();
+  }
+  if (!P->coarse) {
+    const BottomSel sel = select_bottom(desc);
+    P->lb = sel.lb;
+    P->bottom_smem = sel.bottom_smem;
+    P->bottom_stage = sel.bottom_stage;
+    P->bc_nd = sel.bc_nd;
+    P->bc_smem = sel.bc_smem;
   }
   *out = P;
   return PF_OK;
@@ -3055,15 +3186,18 @@ int pf_mg_plan_destroy(pf_mg_plan* P) {
 int pf_mg_bottom_info(const pf_mg_plan* P, int32_t* first_level, int32_t* cluster_levels, int32_t* dense) {
   PF_REQUIRE(P && first_level && cluster_levels && dense, "null argument");
   *first_level = P->lb;
-  *cluster_levels = P->bc_nd;
-  *dense = P->dense_nb > 0 ? 1 : 0;
+  *cluster_levels = P->coarse ? (P->cc.C > 1 ? P->cc.nl : 0) : P->bc_nd;
+  *dense = P->coarse && P->cc.nb > 0 ? 1 : 0;
   return PF_OK;
 }
 
 int64_t pf_mg_bottom_op_floats(const pf_mg_desc* desc) {
   if (!desc || desc->nlev < 1 || desc->nlev > PF_MG_MAX_LEVELS) return 0;
-  const BottomSel sel = select_bottom(desc);
-  return sel.dense_nb > 0 ? (int64_t)sel.dense_nb * sel.dense_nb : 0;
+  CcArgs a;
+  int nq, l0;
+  size_t smem;
+  if (select_coarse(desc, &a, &nq, &smem, &l0) < 0) return 0;
+  return (int64_t)a.nb * a.nb * (desc->precision != PF_PREC_FP32 ? 2 : 1);
 }
 
 int pf_mg_build_hierarchy(pf_mg_plan* P, const float* bx, const float* by, const float* bz, void* stream) {
