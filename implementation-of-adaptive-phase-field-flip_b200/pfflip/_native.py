@@ -98,6 +98,9 @@ SIGNATURES = {
                                                                           C.POINTER(_F), _I32, _I32, _VP, _VP,
                                                                           C.c_size_t, _VP]),
     "pf_particle_max_speed": (C.c_int, [_I64, _VP, _VP, _VP, _VP]),
+    "pf_pack_particles": (C.c_int, [_I64] + [_VP] * 5 + [_VP]),
+    "pf_unpack_particles": (C.c_int, [_I64] + [_VP] * 5 + [_VP]),
+    "pf_gather_particles": (C.c_int, [_I64] + [_VP] * 5 + [_VP]),
     "pf_droplet_classify": (C.c_int, [_G, _I64, _VP, _VP, _VP, _VP, _F, _F, _F, _F, _F, C.c_uint32, _VP, _VP]),
     "pf_velocity_gradient": (C.c_int, [_G, _VP, _VP, _VP, _VP, _VP]),
     "pf_spray_emit": (C.c_int, [_G, _I64, _VP, _VP, _VP, _VP, _VP, _F, _F, _F, _F, _F, _F, C.c_uint32, _VP, _VP]),

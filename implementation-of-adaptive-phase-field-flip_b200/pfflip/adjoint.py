@@ -86,18 +86,18 @@ class DiffSim:
 
     def _to_ids(self, a4):
         """(n, 3) tensor in the caller's order from a float4 stream in array order."""
-        ids = self.sim._ids().long()
         out = torch.empty((self.n, 3), dtype=torch.float32, device=self.sim.dev)
-        out[ids] = a4[:, :3]
+        if self.n:
+            N.call("pf_unpack_particles", self.n, N.sptr(self.sim._vel4), N.sptr(a4), out.data_ptr(), None, None,
+                   N.stream())
         return out
 
-    def _from_ids(self, g, out4):
-        """float4 stream in array order from an (n, 3) tensor in the caller's order."""
-        ids = self.sim._ids().long()
-        out4.zero_()
-        if g is not None:
-            out4[:, :3] = g.to(torch.float32)[ids]
-        return out4
+    def _from_ids(self, gx, gv, gx4, gv4):
+        """float4 streams in array order from (n, 3) tensors in the caller's order
+        (None: zero)."""
+        gx, gv = (None if g is None else g.to(device=self.sim.dev, dtype=torch.float32).contiguous() for g in (gx, gv))
+        N.call("pf_gather_particles", self.n, N.sptr(self.sim._vel4), N.ptr(gx), N.sptr(gx4), N.ptr(gv), N.sptr(gv4),
+               N.stream())
 
     def _grid_stages(self):
         """One step's forward grid stages on the current particles: sort, P2G,
@@ -188,8 +188,7 @@ class DiffSim:
             snaps.append(self._snapshot())
             s._g2p_advect(self.dt, do_g2p=True, do_advect=True)
         ga, gb = self._g4[0], self._g4[1]
-        self._from_ids(gx, ga)
-        self._from_ids(gv, gb)
+        self._from_ids(gx, gv, ga, gb)
         for k in range(nsteps - 1, -1, -1):
             self._restore(snaps[k])
             snaps[k] = None

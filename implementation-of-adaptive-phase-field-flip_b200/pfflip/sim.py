@@ -244,21 +244,16 @@ class Simulator:
             for d, _ in staged.values():
                 d.record_stream(main)
             (dpos, ep), (dvel, ev), (dpt, et) = staged["p"], staged["v"], staged["t"]
-        else:
-            dpos, dvel, dpt = pos.to(dev), vel.to(dev), ptype.to(dev)
-            ep = ev = et = None
-        if ep is not None:
-            main.wait_event(ep)
-        p4[:, :3].copy_(dpos)
-        if ev is not None:
-            main.wait_event(ev)
-        v4[:, :3].copy_(dvel)
-        if et is not None:
+            # the liquid flag is formed on the device: a host-side comparison would
+            # be a CPU pass over n values and an unpinned copy
             main.wait_event(et)
-        # the liquid flag is formed on the device: a host-side comparison would
-        # be a CPU pass over n values and an unpinned copy
-        p4.view(torch.int32)[:, 3].copy_((dpt == 1).to(torch.int32))
-        v4.view(torch.int32)[:, 3] = torch.arange(n, dtype=torch.int32, device=dev)
+            main.wait_event(ep)
+            N.call("pf_pack_particles", n, N.ptr(dpos), N.ptr(dpt), N.sptr(p4), None, None, N.stream())
+            main.wait_event(ev)
+            N.call("pf_pack_particles", n, None, None, None, N.ptr(dvel), N.sptr(v4), N.stream())
+        else:
+            dpos, dvel, dpt = (a.to(dev).contiguous() for a in (pos, vel, ptype))
+            N.call("pf_pack_particles", n, N.ptr(dpos), N.ptr(dpt), N.sptr(p4), N.ptr(dvel), N.sptr(v4), N.stream())
         if self.cfg.droplets:
             self._drop_r.zero_()
         self._sort()
@@ -282,14 +277,24 @@ class Simulator:
         they have landed; handing them straight back to set_particles is safe,
         which is what lets a host round trip per step overlap its uploads with
         the downloads."""
-        ids = self._ids().long()
         main = torch.cuda.current_stream(self.dev)
         out = []
         copied = False
         pending = []
+        n = self.n_particles
+
+        def direct(d):  # a device tensor that takes the rows as they are
+            return (d is not None and d.device == self.dev and d.dtype == torch.float32 and d.is_contiguous()
+                    and d.shape == (n, 3))
+
+        if direct(pos_out) and direct(vel_out):
+            N.call("pf_unpack_particles", n, N.sptr(self._vel4), N.sptr(self._pos4), N.ptr(pos_out),
+                   N.sptr(self._vel4), N.ptr(vel_out), N.stream())
+            self._pending_d2h = []
+            return pos_out, vel_out
         for src, dst in ((self._pos4, pos_out), (self._vel4, vel_out)):
-            tmp = torch.empty((self.n_particles, 3), dtype=torch.float32, device=self.dev)
-            tmp[ids] = src[:, :3]
+            tmp = torch.empty((n, 3), dtype=torch.float32, device=self.dev)
+            N.call("pf_unpack_particles", n, N.sptr(self._vel4), N.sptr(src), tmp.data_ptr(), None, None, N.stream())
             if dst is None:
                 out.append(tmp.cpu())
             elif dst.device.type == "cpu" and dst.is_contiguous():

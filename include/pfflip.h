@@ -215,6 +215,18 @@ int pf_g2p_advect_packed(const pf_grid* g, int64_t n, float* pos4, float* vel4, 
  * replaces pfflip/kernels.py:552-564 (particle_max_speed). */
 int pf_particle_max_speed(int64_t n, const float* pos4, const float* vel4, float* out, void* stream);
 
+/* The caller's (n, 3) arrays and the float4 streams (no reference counterpart:
+ * the reference keeps plain arrays).  pack: pos4 = (pos, flags: type == 1) and
+ * vel4 = (vel, index); pos4 or vel4 may be NULL.  unpack: rows of the streams
+ * a4 and b4 (in the order of vel4) to a[index], b[index]; a or b may be NULL.
+ * gather: a4 = (a[index], 0), b4 = (b[index], 0), zero where a or b is NULL. */
+int pf_pack_particles(int64_t n, const float* pos, const int32_t* type, float* pos4, const float* vel, float* vel4,
+                      void* stream);
+int pf_unpack_particles(int64_t n, const float* vel4, const float* a4, float* a, const float* b4, float* b,
+                        void* stream);
+int pf_gather_particles(int64_t n, const float* vel4, const float* a, float* a4, const float* b, float* b4,
+                        void* stream);
+
 /* ------------------------------------------------------------- droplets */
 /* Escaped particles, droplets and spray; pfflip/droplets.py as run by
  * pfflip/sim.py:343-401.  A particle's state is bits 1-2 of its flags

@@ -1,0 +1,51 @@
+"""Particle state in and out of the simulator: set_particles and read_particles
+against the arrays themselves (copies: the tolerance is zero), for counts around
+a warp and a block, every kind of source (host, device, strided, other dtypes)
+and of destination (device, strided device, host, none)."""
+
+import numpy as np
+import pytest
+import torch
+
+from pfflip import Config, Simulator
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def state(n):
+    rng = np.random.default_rng(n + 1)
+    pos = rng.random((n, 3), dtype=np.float32)
+    vel = rng.standard_normal((n, 3)).astype(np.float32)
+    return pos, vel, rng.integers(0, 3, n).astype(np.int32)  # type 2 is not liquid
+
+
+def sources(kind, pos, vel, typ):
+    if kind == "host":
+        return pos, vel, typ
+    t = [torch.from_numpy(a).to(DEV) for a in (pos, vel, typ)]
+    if kind == "strided":
+        wide = [torch.zeros(len(pos), 7, device=DEV) for _ in range(2)]
+        for w, a in zip(wide, t):
+            w[:, 1:6:2] = a
+        return wide[0][:, 1:6:2], wide[1][:, 1:6:2], t[2].repeat_interleave(2)[::2]
+    if kind == "double":
+        return t[0].double(), t[1].double(), t[2].long()
+    return t
+
+
+@pytest.mark.parametrize("kind", ["host", "device", "strided", "double"])
+@pytest.mark.parametrize("n", [0, 1, 31, 257, 5000])
+def test_particles_round_trip(n, kind):
+    pos, vel, typ = state(n)
+    sim = Simulator(Config(res=(6, 5, 4), dx=0.25, ppc=8, droplets=False, device=DEV))
+    sim.set_particles(*sources(kind, pos, vel, typ))
+    assert np.array_equal(sim.ptype.numpy(), (typ == 1).astype(np.int32))
+    outs = [(None, None), tuple(torch.empty(n, 3, device=DEV) for _ in range(2)),
+            tuple(torch.empty(n, 6, device=DEV)[:, ::2] for _ in range(2)),
+            tuple(torch.empty(n, 3) for _ in range(2)), (None, torch.empty(n, 3, device=DEV))]
+    for po, vo in outs:
+        x, v = sim.read_particles(po, vo)
+        assert (po is None or x is po) and (vo is None or v is vo)
+        torch.cuda.synchronize()
+        assert np.array_equal(x.cpu().numpy(), pos) and np.array_equal(v.cpu().numpy(), vel)
