@@ -2171,6 +2171,9 @@ struct pf_mg_plan {
   size_t cc_smem;
   pf::CcArgs cc;       // geometry; the pointers are set per launch
   int dense_l0;        // first level of the dense operator (cc.nb > 0)
+  bool whole;          // k_solve runs the solve: k_coarse covers every level and the CG vectors fit (args in cs)
+  size_t cs_smem;
+  pf::CcSolveArgs cs;  // offsets; cc is taken from above
   cudaStream_t cap_stream;
   cudaGraphExec_t exec[2];
   size_t exec_nodes[2];
@@ -2435,6 +2438,10 @@ int launch_bottom_cluster(pf_mg_plan* P, const TB* b, const float* b_scale, bool
   return PF_OK;
 }
 
+template <class T> void* solve_kernel(int nq) {
+  return nq <= 1 ? (void*)k_solve<T, 1> : nq <= 2 ? (void*)k_solve<T, 2> : (void*)k_solve<T, 3>;
+}
+
 template <class T> void* coarse_kernel(int nq) {
   return nq <= 1 ? (void*)k_coarse<T, 1> : nq <= 2 ? (void*)k_coarse<T, 2> : (void*)k_coarse<T, 3>;
 }
@@ -2455,10 +2462,9 @@ cudaLaunchConfig_t coarse_config(int C, size_t smem, cudaStream_t s, cudaLaunchA
   return cfg;
 }
 
-template <class T, class TB>
-int launch_coarse(pf_mg_plan* P, const TB* b, const float* b_scale, bool want_mean, cudaStream_t s, T** out) {
+// the cluster kernels' arguments for a right-hand side (no scale)
+template <class T, class TB> CcArgs coarse_args(pf_mg_plan* P, const TB* b) {
   CcArgs a = P->cc;
-  LV<T> V0 = view<T>(P, P->lb);
   for (int l = 0; l < a.nl; ++l) {
     LV<T> V = view<T>(P, P->lb + l);
     a.L[l].bx = V.bx;
@@ -2468,8 +2474,6 @@ int launch_coarse(pf_mg_plan* P, const TB* b, const float* b_scale, bool want_me
   a.M = P->d.bottom_op;
   a.b = b;
   a.b_f32 = std::is_same<TB, float>::value ? 1 : 0;
-  a.b_scale = b_scale;
-  a.p_out = V0.p0;
   a.omega = P->d.omega;
   a.pre = P->d.pre;
   a.post = P->d.post;
@@ -2478,8 +2482,17 @@ int launch_coarse(pf_mg_plan* P, const TB* b, const float* b_scale, bool want_me
   a.pscale = mixed(P) ? 2.f : 1.f;
   a.flux = FLUX(P);
   a.st = ST(P);
-  a.want_mean = want_mean ? 1 : 0;
   a.mixed = mixed(P) ? 1 : 0;
+  return a;
+}
+
+template <class T, class TB>
+int launch_coarse(pf_mg_plan* P, const TB* b, const float* b_scale, bool want_mean, cudaStream_t s, T** out) {
+  CcArgs a = coarse_args<T, TB>(P, b);
+  LV<T> V0 = view<T>(P, P->lb);
+  a.b_scale = b_scale;
+  a.p_out = V0.p0;
+  a.want_mean = want_mean ? 1 : 0;
   cudaLaunchAttribute attr[2];
   const cudaLaunchConfig_t cfg = coarse_config(a.C, P->cc_smem, s, attr);
   void* args[] = {&a};
@@ -2722,34 +2735,65 @@ template <class T> int capture_graphs(pf_mg_plan* P) {
   return PF_OK;
 }
 
+// the whole solve in one launch of the cluster kernel
+template <class T> int enqueue_whole(pf_mg_plan* P, const float* b, float* x, float tol, int max_iter, cudaStream_t s) {
+  CcSolveArgs A = P->cs;
+  A.cc = coarse_args<T, float>(P, b);
+  A.x = x;
+  A.tol = tol;
+  A.max_iter = max_iter;
+  A.coef_scale = P->d.coef_scale;
+  A.bx = P->d.lev[0].bx;
+  A.by = P->d.lev[0].by;
+  A.bz = P->d.lev[0].bz;
+  A.n_total = (int)ncells(P->d.lev[0]);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = coarse_config(A.cc.C, P->cs_smem, s, attr);
+  cfg.numAttrs = 1;  // the operator it stages first may come from the kernel before it
+  void* args[] = {&A};
+  PF_CUDA_TRY(cudaLaunchKernelExC(&cfg, solve_kernel<T>(P->cc_nq), args));
+  PF_LAUNCHED();
+  return PF_OK;
+}
+
+// Iterations one launch may run: an iteration takes 15 to 60 us, so a launch ends
+// within 0.1 s.  Longer solves, and verbose ones (a line per iteration), launch
+// every iteration.
+constexpr int kWholeMaxIter = 1000;
+
 template <class T>
 int solve_impl(pf_mg_plan* P, const float* b, float* x, float tol, int max_iter, int use_graphs, int verbose,
                int* iters_out, double* rel_out, cudaStream_t s) {
-  PF_TRY(enqueue_setup<T>(P, b, tol, max_iter, s));
-  if (use_graphs && !P->graphs_ready) PF_TRY(capture_graphs<T>(P));
-  for (int k = 1; k <= max_iter; ++k) {
-    const int par = (k - 1) & 1;
-    if (use_graphs) {
-      PF_CUDA_TRY(cudaGraphLaunch(P->exec[par], s));
-      count_launch(P->exec_nodes[par]);
-    } else {
-      PF_TRY(enqueue_iteration<T>(P, par, s));
+  const bool whole = P->whole && !verbose && max_iter <= kWholeMaxIter;
+  if (whole) {
+    PF_TRY(enqueue_whole<T>(P, b, x, tol, max_iter, s));
+  } else {
+    PF_TRY(enqueue_setup<T>(P, b, tol, max_iter, s));
+    if (use_graphs && !P->graphs_ready) PF_TRY(capture_graphs<T>(P));
+    for (int k = 1; k <= max_iter; ++k) {
+      const int par = (k - 1) & 1;
+      if (use_graphs) {
+        PF_CUDA_TRY(cudaGraphLaunch(P->exec[par], s));
+        count_launch(P->exec_nodes[par]);
+      } else {
+        PF_TRY(enqueue_iteration<T>(P, par, s));
+      }
+      PF_CUDA_TRY(cudaMemcpyAsync(P->h_state[k & 1], P->d.state, sizeof(MGState), cudaMemcpyDeviceToHost, s));
+      PF_CUDA_TRY(cudaEventRecord(P->ev[k & 1], s));
+      if (verbose) {
+        PF_CUDA_TRY(cudaEventSynchronize(P->ev[k & 1]));
+        const MGState* h = P->h_state[k & 1];
+        if (h->it == k) std::printf("    pcg it=%3d  |r|inf/|b|inf = %.3e\n", h->it, h->rel);
+        if (h->done) break;
+        continue;
+      }
+      if (k >= 2) {
+        PF_CUDA_TRY(cudaEventSynchronize(P->ev[(k - 1) & 1]));
+        if (P->h_state[(k - 1) & 1]->done) break;
+      }
     }
-    PF_CUDA_TRY(cudaMemcpyAsync(P->h_state[k & 1], P->d.state, sizeof(MGState), cudaMemcpyDeviceToHost, s));
-    PF_CUDA_TRY(cudaEventRecord(P->ev[k & 1], s));
-    if (verbose) {
-      PF_CUDA_TRY(cudaEventSynchronize(P->ev[k & 1]));
-      const MGState* h = P->h_state[k & 1];
-      if (h->it == k) std::printf("    pcg it=%3d  |r|inf/|b|inf = %.3e\n", h->it, h->rel);
-      if (h->done) break;
-      continue;
-    }
-    if (k >= 2) {
-      PF_CUDA_TRY(cudaEventSynchronize(P->ev[(k - 1) & 1]));
-      if (P->h_state[(k - 1) & 1]->done) break;
-    }
+    PF_TRY(enqueue_final(P, x, s));
   }
-  PF_TRY(enqueue_final(P, x, s));
   PF_CUDA_TRY(cudaMemcpyAsync(P->h_state[0], P->d.state, sizeof(MGState), cudaMemcpyDeviceToHost, s));
   PF_CUDA_TRY(cudaStreamSynchronize(s));
   const MGState* h = P->h_state[0];
@@ -2858,6 +2902,8 @@ template <class T> cudaError_t set_smem_attrs() {
   for (int nq : {1, 2, 3}) {
     chk(cudaFuncSetAttribute(coarse_kernel<T>(nq), cudaFuncAttributeMaxDynamicSharedMemorySize, kCcSmemMax));
     chk(cudaFuncSetAttribute(coarse_kernel<T>(nq), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    chk(cudaFuncSetAttribute(solve_kernel<T>(nq), cudaFuncAttributeMaxDynamicSharedMemorySize, kCcSmemMax));
+    chk(cudaFuncSetAttribute(solve_kernel<T>(nq), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   }
   chk(cudaFuncSetAttribute(k_rb_tile<T, float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
   chk(cudaFuncSetAttribute(k_rb_tile<T, T, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
@@ -3158,6 +3204,23 @@ int pf_mg_plan_create(const pf_mg_desc* desc, pf_mg_plan** out) {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) P->coarse = false;
     cudaGetLastError();
+  }
+  if (P->coarse && P->lb == 0) {
+    // the CG vectors behind k_coarse's shared memory
+    const CcLevel& L = P->cc.L[0];
+    size_t off = P->cc_smem / sizeof(float);
+    auto take = [&off](size_t floats) {
+      const size_t o = off;
+      off += (floats + 3) / 4 * 4;
+      return (int)o;
+    };
+    P->cs.oQ = take(2 * (size_t)(L.smax + 2) * L.n1 * L.hk);
+    const size_t v = 4 * (size_t)(P->cc_nq <= 3 ? P->cc_nq : 3) * CC_NT;
+    P->cs.oR = take(v);
+    P->cs.oR2 = take(v);
+    P->cs.oX = take(v);
+    P->cs_smem = off * sizeof(float);
+    P->whole = P->cs_smem <= (size_t)kCcSmemMax;
   }
   if (!P->coarse) {
     const BottomSel sel = select_bottom(desc);

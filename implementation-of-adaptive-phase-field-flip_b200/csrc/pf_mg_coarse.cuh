@@ -194,6 +194,8 @@ template <class T, int NQ> struct CoarseCycle {
   unsigned turn;   // halo exchanges so far, on any level
   unsigned phase;  // phase bits of the four mbarriers
   bool fail;       // a wait ran out: no more waits, the result is flagged
+  unsigned bvec;   // shared address of the top level's right-hand side (0: a.b), and its scale
+  float bvec_scale;
   // the level at hand
   int pl, cnt, s, lo, hk;
   unsigned P[2];      // shared addresses of the red and black arrays
@@ -210,6 +212,8 @@ template <class T, int NQ> struct CoarseCycle {
     held = -1;
     turn = phase = par = 0u;
     fail = false;
+    bvec = 0u;
+    bvec_scale = 1.f;
   }
 
   __device__ __forceinline__ bool on(int u) const { return u * CC_NT + tid < cnt; }
@@ -257,13 +261,15 @@ template <class T, int NQ> struct CoarseCycle {
   // of the domain counts in the diagonal and has no neighbour
   __device__ __forceinline__ void load_coefs(int l) {
     if (held == l || s == 0) return;
-    held = l;
-    par = 0u;
     const CcLevel& L = a.L[l];
+    load_faces(L, reinterpret_cast<const T*>(L.bx), reinterpret_cast<const T*>(L.by), reinterpret_cast<const T*>(L.bz));
+    held = l;
+  }
+
+  template <class F> __device__ __forceinline__ void load_faces(const CcLevel& L, const F* X, const F* Y, const F* Z) {
+    held = -1;
+    par = 0u;
     const int n0 = L.n0, n1 = L.n1, n2 = L.n2;
-    const T* X = reinterpret_cast<const T*>(L.bx);
-    const T* Y = reinterpret_cast<const T*>(L.by);
-    const T* Z = reinterpret_cast<const T*>(L.bz);
     const bool wide = (n2 & 3) == 0 && ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Y)) & 15u) == 0;
 #pragma unroll
     for (int u = 0; u < NQ; ++u) {
@@ -279,9 +285,9 @@ template <class T, int NQ> struct CoarseCycle {
         j = row - li * n1;
         i = lo + li;
         const int r = i * n1 + j;
-        const T* x = X + r * n2 + 4 * h;
-        const T* y = Y + (r + i) * n2 + 4 * h;
-        const T* zz = Z + r * (n2 + 1) + 4 * h;
+        const F* x = X + r * n2 + 4 * h;
+        const F* y = Y + (r + i) * n2 + 4 * h;
+        const F* zz = Z + r * (n2 + 1) + 4 * h;
         if (wide) {
           cc_ld4(x, xl);
           cc_ld4(x + n1 * n2, xu);
@@ -337,6 +343,14 @@ template <class T, int NQ> struct CoarseCycle {
   // the right-hand side of the level's quads: from global memory (top), or the
   // two plane sums the level above left in the slots
   __device__ __forceinline__ void load_b(int l) {
+    if (l == 0 && bvec != 0u) {
+      const f2 sc = f2_bcast(bvec_scale);
+#pragma unroll
+      for (int u = 0; u < NQ; ++u)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) b[c][u] = f2_mul(vec(bvec, c, u), sc);
+      return;
+    }
     const CcLevel& L = a.L[l];
     const float bsc = l == 0 && a.b_scale ? *a.b_scale : 1.f;
     const size_t g0 = (size_t)lo * L.n1 * L.n2;
@@ -380,6 +394,12 @@ template <class T, int NQ> struct CoarseCycle {
       b[1][u] = o ? f2_make(v[u][0], v[u][2]) : f2_make(v[u][1], v[u][3]);
     }
   }
+
+  // a vector of the top level's cells private to their threads: f2 per colour and quad
+  __device__ __forceinline__ unsigned vec_at(unsigned v, int c, int u) const {
+    return v + 8u * (unsigned)((c * NQ + u) * CC_NT + tid);
+  }
+  __device__ __forceinline__ f2 vec(unsigned v, int c, int u) const { return cc_lds2(vec_at(v, c, u)); }
 
   // p of the level's quads from the shared arrays
   __device__ __forceinline__ void load_p() {
@@ -885,6 +905,337 @@ __global__ void __launch_bounds__(CC_NT, 1) k_coarse(const __grid_constant__ CcA
     a.st->status = ST_TMA_TIMEOUT;
     a.st->done = 1;
   }
+}
+
+// ---------------------------------------------------------------- the whole solve in the cluster
+// Where k_coarse covers every level, the flexible CG around it runs in the same
+// launch: r, x and A q stay in shared memory private to the threads that own
+// the cells, q in two colour arrays with halo planes like p, the scalars in
+// every thread.  An iteration is then the V-cycle and three reductions (q A q,
+// max|r|, and the mean of z together with the dot products, since
+// <r, z + c> = <r, z> + c <r, 1>) instead of six launches and a copy back.
+// Sums are FP64 per thread, combined in a fixed order; the update formulas are
+// those of the launched path (pfflip/poisson.py:355-409).
+//
+// Bound by the same chains as k_coarse, plus about 1 us a reduction.  Measured on
+// a B200 against the launched CG around k_coarse, us: 32^3 solve to 1e-4 829 ->
+// 555, four 16^3 steps 2924 -> 1938, a 24^3 gradient of two steps 6700 -> 4664.
+constexpr int CC_RED = 4;  // values reduced at once
+
+struct CcSolveArgs {
+  CcArgs cc;
+  float* x;        // solution, mean removed
+  float tol;
+  int max_iter;
+  float coef_scale;
+  const float* bx;  // FP32 faces of the top level: the CG's operator
+  const float* by;
+  const float* bz;
+  int n_total;
+  int oQ;          // q: colour arrays with halos, as level 0's p
+  int oR, oR2, oX; // vectors of f2 (16-byte aligned)
+};
+
+template <class T, int NQ>
+__global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSolveArgs A) {
+  extern __shared__ __align__(16) float ccsm[];
+  __shared__ double sred[40];
+  __shared__ double s_part[CC_MAXC + 1];
+  __shared__ double s_warp[CC_RED][CC_NT / 32];
+  __shared__ double s_all[2][CC_RED][CC_MAXC];
+  __shared__ int s_go[2];
+  const CcArgs& a = A.cc;
+  CoarseCycle<T, NQ> cy(a, ccsm);
+  const int tid = cy.tid;
+  const CcLevel& L = a.L[0];
+  cy.stage_dense();
+  cy.init_barriers();
+  for (int l = 0; l < a.nl; ++l) {
+    cy.enter(l);
+    if (cy.s > 0) {
+      cy.load_coefs(l);
+      break;
+    }
+  }
+  const int nq4 = (L.smax + 2) * L.n1 * L.hk / 2;  // q: 2 (smax + 2) n1 hk floats
+  auto rezero = [&]() {
+    for (int e = tid; e < a.zero_floats / 4; e += CC_NT)
+      reinterpret_cast<float4*>(ccsm)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  rezero();
+  for (int e = tid; e < nq4; e += CC_NT) reinterpret_cast<float4*>(ccsm + A.oQ)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+
+  // sums (MAX: maxima) of K per-thread values over the top level's CTAs, in
+  // every thread that needs them: those CTAs (A == 1), or all of the cluster
+  unsigned red_turn = 0;
+  auto reduce = [&](auto kc, auto is_max, double (&v)[CC_RED]) {
+    constexpr int K = decltype(kc)::value;
+    constexpr bool MAX = decltype(is_max)::value;
+    const int lane = tid & 31, w = tid >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      double t = v[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double q = __shfl_xor_sync(0xffffffffu, t, o);
+        t = MAX ? fmax(t, q) : t + q;
+      }
+      if (lane == 0) s_warp[k][w] = t;
+    }
+    __syncthreads();
+    const unsigned buf = red_turn++ & 1u;
+    if (w < K) {
+      double t = lane < CC_NT / 32 ? s_warp[w][lane] : 0.0;
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        const double q = __shfl_xor_sync(0xffffffffu, t, o);
+        t = MAX ? fmax(t, q) : t + q;
+      }
+      if (L.A == 1) {
+        if (lane == 0) s_all[buf][w][0] = t;
+      } else if (cy.s > 0 && lane < a.C) {
+        cc_st(cc_map(smem_u32(&s_all[buf][w][cy.rank - L.c0]), lane), t);
+      }
+    }
+    if (L.A == 1) __syncthreads();
+    else cc_sync();
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      double t = s_all[buf][k][0];
+      for (int r = 1; r < L.A; ++r) t = MAX ? fmax(t, s_all[buf][k][r]) : t + s_all[buf][k][r];
+      v[k] = t;
+    }
+  };
+  auto k1 = std::integral_constant<int, 1>();
+  auto k4 = std::integral_constant<int, 4>();
+  auto sum = std::false_type();
+  auto mx = std::true_type();
+  // the decision of the top level's CTAs, known to the cluster
+  unsigned go_turn = 0;
+  auto agree = [&](bool go) {
+    if (L.A > 1 || a.C == 1) return go;
+    const unsigned buf = go_turn++ & 1u;
+    if (cy.s > 0 && tid < a.C) {
+      unsigned at = cc_map(smem_u32(&s_go[buf]), tid);
+      asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(at), "r"(go ? 1 : 0) : "memory");
+    }
+    cc_sync();
+    return s_go[buf] != 0;
+  };
+
+  if (a.C > 1) cc_sync();
+  else __syncthreads();
+  cy.enter(0);
+  const bool mine = cy.s > 0;
+  const unsigned sm0 = cy.sm0, Rv[2] = {sm0 + 4u * (unsigned)A.oR, sm0 + 4u * (unsigned)A.oR2};
+  const unsigned Xv = sm0 + 4u * (unsigned)A.oX;
+  int cur = 0;
+  unsigned in = 0u;  // bit 4 u + 2 c + d: cell d of colour c of quad u exists
+  double red[CC_RED];
+
+  // ---- r = b - mean(b), x = 0, |b|   (pfflip/poisson.py:363-372)
+  red[0] = 0.0;
+  if (mine) {
+    cy.load_b(0);
+#pragma unroll
+    for (int u = 0; u < NQ; ++u)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        bool e[2] = {false, false};
+        if (cy.on(u)) cy.present(L, u, c, e);
+        in |= (e[0] ? 1u : 0u) << (4 * u + 2 * c) | (e[1] ? 2u : 0u) << (4 * u + 2 * c);
+        red[0] += (double)f2_x(cy.b[c][u]) + (double)f2_y(cy.b[c][u]);
+      }
+  }
+  auto masked = [&](int c, int u, float x, float y) {
+    const unsigned m = in >> (4 * u + 2 * c);
+    return f2_make(m & 1u ? x : 0.f, m & 2u ? y : 0.f);
+  };
+  auto amax = [](float x, float m) { return fmaxf(m, isfinite(x) ? fabsf(x) : INFINITY); };
+  reduce(k1, sum, red);
+  const double n = (double)A.n_total;
+  float m = 0.f;
+  {
+    const float c0 = (float)(-(red[0] / n));
+#pragma unroll
+    for (int u = 0; u < NQ; ++u)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (!mine || !cy.on(u)) continue;
+        const f2 r = masked(c, u, f2_x(cy.b[c][u]) + c0, f2_y(cy.b[c][u]) + c0);
+        m = amax(f2_x(r), m);
+        m = amax(f2_y(r), m);
+        cc_sts2(cy.vec_at(Rv[0], c, u), r);
+        cc_sts2(cy.vec_at(Xv, c, u), f2_bcast(0.f));
+      }
+  }
+  red[0] = (double)m;
+  reduce(k1, mx, red);
+  const double bnorm = red[0];
+  double rel = 1.0, rz = 0.0, sum_r_old = 0.0;
+  int it = 0, status = ST_RUNNING;
+  bool go = A.max_iter > 0;
+  if (!(bnorm > 0.0) || isinf(bnorm)) {
+    status = bnorm == 0.0 ? ST_ZERO_RHS : ST_NONFINITE;
+    rel = bnorm == 0.0 ? 0.0 : 1.0;
+    go = false;
+  }
+  // 16-bit hierarchy: the top right-hand side is r * scale_r, a power of two
+  // putting max|r| in [0.5, 1)
+  float scale_r = 1.f;
+  auto rescale = [&](double mr) {
+    int ex = 0;
+    frexpf(mr > 0.0 ? (float)mr : 1.f, &ex);
+    if (a.mixed) scale_r = ldexpf(1.f, -ex);
+  };
+  rescale(bnorm);
+  bool first = true;
+  while (agree(go)) {
+    // ---- z = V-cycle(r) with its mean removed
+    cy.bvec = Rv[cur];
+    cy.bvec_scale = scale_r;
+    cy.enter(0);
+    if (mine) {
+      cy.load_coefs(0);
+      cy.load_b(0);
+    }
+    cy.cycle(sred, s_part);
+    __syncthreads();
+    rezero();  // for the next cycle; a reduction or a cluster barrier comes first
+    cy.enter(0);
+    const float zs = a.mixed ? A.coef_scale / scale_r : 1.f;
+#pragma unroll
+    for (int k = 0; k < CC_RED; ++k) red[k] = 0.0;
+#pragma unroll
+    for (int u = 0; u < NQ; ++u)
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        if (!mine || !cy.on(u)) continue;
+        const f2 p = masked(c, u, roundT<T>(f2_x(cy.p[c][u])) * zs, roundT<T>(f2_y(cy.p[c][u])) * zs);
+        const f2 rn = cy.vec(Rv[cur], c, u), ro = cy.vec(Rv[cur ^ 1], c, u);
+        cy.p[c][u] = p;
+        const double px = f2_x(p), py = f2_y(p);
+        red[0] += px + py;
+        red[1] += (double)f2_x(rn) * px + (double)f2_y(rn) * py;
+        if (!first) red[2] += (double)f2_x(ro) * px + (double)f2_y(ro) * py;
+        red[3] += (double)f2_x(rn) + (double)f2_y(rn);
+      }
+    reduce(k4, sum, red);
+    const float cs = (float)(-(red[0] / n));
+    const double rz_new = red[1] + (double)cs * red[3], rpz = red[2] + (double)cs * sum_r_old;
+    const float beta = first || rz == 0.0 ? 0.f : (float)fmax((rz_new - rpz) / rz, 0.0);
+    rz = rz_new;
+    sum_r_old = red[3];
+    // ---- q = z + beta q, A q, <q, A q>
+    cy.P[0] = sm0 + 4u * (unsigned)A.oQ;
+    cy.P[1] = cy.P[0] + 4u * (unsigned)((L.smax + 2) * cy.pl);
+    red[0] = 0.0;
+    if (mine) {
+      f2 q0[NQ], q1[NQ];
+#pragma unroll
+      for (int u = 0; u < NQ; ++u) {
+        q0[u] = q1[u] = f2_bcast(0.f);
+        if (!cy.on(u)) continue;
+        const f2 o0 = cc_lds2(cy.P[0] + 4u * cy.at(u)), o1 = cc_lds2(cy.P[1] + 4u * cy.at(u));
+        q0[u] = masked(0, u, (f2_x(cy.p[0][u]) + cs) + beta * f2_x(o0), (f2_y(cy.p[0][u]) + cs) + beta * f2_y(o0));
+        q1[u] = masked(1, u, (f2_x(cy.p[1][u]) + cs) + beta * f2_x(o1), (f2_y(cy.p[1][u]) + cs) + beta * f2_y(o1));
+        cy.b[0][u] = cy.b[1][u] = f2_bcast(0.f);
+      }
+      cy.template put<0>(q0, true);
+      cy.template put<1>(q1, true);
+      // the 16-bit coefficients give way to the FP32 ones for this product
+      if (!std::is_same<T, float>::value) cy.load_faces(L, A.bx, A.by, A.bz);
+      cy.settle(2);
+      cy.template residual<0>(q0);  // - A q
+      cy.template residual<1>(q1);
+#pragma unroll
+      for (int u = 0; u < NQ; ++u) {
+        if (!cy.on(u)) continue;
+        red[0] -= (double)f2_x(cy.p[0][u]) * (double)f2_x(q0[u]) + (double)f2_y(cy.p[0][u]) * (double)f2_y(q0[u]);
+        red[0] -= (double)f2_x(cy.p[1][u]) * (double)f2_x(q1[u]) + (double)f2_y(cy.p[1][u]) * (double)f2_y(q1[u]);
+        // the older residual is used up: its place takes - A q, then the new one
+        cc_sts2(cy.vec_at(Rv[cur ^ 1], 0, u), q0[u]);
+        cc_sts2(cy.vec_at(Rv[cur ^ 1], 1, u), q1[u]);
+      }
+    } else {
+      cy.turn += 2u;
+    }
+    reduce(k1, sum, red);
+    const double qAq = red[0];
+    ++it;
+    first = false;
+    if (!(qAq > 0.0)) {
+      status = qAq <= 0.0 ? ST_BREAKDOWN : ST_NONFINITE;
+      go = false;
+    }
+    // ---- x += alpha q, r -= alpha A q, |r|   (pfflip/poisson.py:390-398)
+    const float al = go ? (float)(rz / qAq) : 0.f;
+    m = 0.f;
+    if (go) {
+#pragma unroll
+      for (int u = 0; u < NQ; ++u)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          if (!mine || !cy.on(u)) continue;
+          const f2 x = cy.vec(Xv, c, u), r = cy.vec(Rv[cur], c, u), Aq = cy.vec(Rv[cur ^ 1], c, u), af = f2_bcast(al);
+          const f2 rn = f2_fma(af, Aq, r);
+          m = amax(f2_x(rn), m);
+          m = amax(f2_y(rn), m);
+          cc_sts2(cy.vec_at(Xv, c, u), f2_fma(af, cy.p[c][u], x));
+          cc_sts2(cy.vec_at(Rv[cur ^ 1], c, u), rn);
+        }
+      cur ^= 1;
+    }
+    red[0] = (double)m;
+    reduce(k1, mx, red);
+    if (go) {
+      rel = red[0] / bnorm;
+      if (!(rel == rel) || isinf(rel)) {
+        status = ST_NONFINITE;
+        go = false;
+      } else if (rel < (double)A.tol) {
+        status = ST_CONVERGED;
+        go = false;
+      }
+      if (it >= A.max_iter) go = false;
+      rescale(red[0]);
+    }
+  }
+
+  // ---- x with its mean removed
+  red[0] = 0.0;
+#pragma unroll
+  for (int u = 0; u < NQ; ++u)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      if (!mine || !cy.on(u)) continue;
+      const f2 x = cy.vec(Xv, c, u);
+      red[0] += (double)f2_x(x) + (double)f2_y(x);
+    }
+  reduce(k1, sum, red);
+  const float cx = (float)(-(red[0] / n));
+  float* out = A.x + (size_t)cy.lo * L.n1 * L.n2;
+#pragma unroll
+  for (int u = 0; u < NQ; ++u) {
+    if (!mine || !cy.on(u)) continue;
+    int row, h;
+    cy.locate(L, u, row, h);
+    const f2 x0 = cy.vec(Xv, cy.odd(u), u), x1 = cy.vec(Xv, 1 - cy.odd(u), u);
+    const float v[4] = {f2_x(x0), f2_x(x1), f2_y(x0), f2_y(x1)};
+#pragma unroll
+    for (int d = 0; d < 4; ++d)
+      if (4 * h + d < L.n2) out[row * L.n2 + 4 * h + d] = v[d] + cx;
+  }
+  if (mine && cy.rank == L.c0 && tid == 0) {
+    a.st->it = it;
+    a.st->rel = rel;
+    a.st->bnorm = bnorm;
+    a.st->status = status;
+    a.st->done = 1;
+  }
+  if (cy.fail) a.st->status = ST_TMA_TIMEOUT;
+  if (a.C > 1) cc_sync();  // no CTA leaves while another may still write to it
 }
 
 }  // namespace pf

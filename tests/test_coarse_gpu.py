@@ -85,3 +85,45 @@ def test_coarse_vcycle_16bit_matches_separate_sweeps(res, precision, monkeypatch
         g, z[mode] = vcycle(res, bx, by, bz, b, pre=2, post=2, precision=precision)
     # bfloat16 keeps 8 bits where binary16 keeps 11
     assert off(z[""], z["cta"]) < (1e-2 if precision == "fp16" else 8e-2)
+
+
+def solves(g, res, b, tol, max_iter):
+    """(iterations, residual, x) of the one-launch solve and of the launched CG
+    (verbose solves take that one)."""
+    out = []
+    for verbose in (False, True):
+        x = DeviceArray.zeros(res, device=DEV)
+        it, rel = g.solve(dev(b), x, tol=tol, max_iter=max_iter, verbose=verbose)
+        out.append((it, rel, x.numpy().astype(np.float64)))
+    return out
+
+
+@pytest.mark.parametrize("precision,stencil,tol", [("fp32", "flux", 1e-6), ("fp32", "reference", 1e-4), ("fp16", "flux", 1e-6)])
+@pytest.mark.parametrize("res", [(4, 4, 4), (16, 16, 16), (13, 11, 9), (21, 23, 27), (20, 20, 22), (32, 32, 32),
+                                 (38, 44, 38), (40, 40, 40)])
+def test_one_launch_solve_matches_launched_cg(res, precision, stencil, tol):
+    """Same iterations within 1; the solutions differ by what the tolerance
+    leaves open, 10 tol of the maximum as in the comparisons with binary64."""
+    bx, by, bz, b, _ = scenes.solve_problem(res, seed=34)
+    g = MGPCG(res, DEV, pre=3, post=3, precision=precision, stencil=stencil)
+    g.build_hierarchy(dev(bx), dev(by), dev(bz))
+    (i1, r1, x1), (i2, r2, x2) = solves(g, res, b, tol, 200)
+    assert r1 < tol and r2 < tol and abs(i1 - i2) <= 1, (i1, r1, i2, r2)
+    assert abs(x1.mean()) < 1e-6 * np.abs(x1).max()
+    assert off(x1, x2) < 10 * tol
+
+
+@pytest.mark.parametrize("res", [(16, 16, 16), (32, 32, 32), (13, 11, 9)])
+def test_one_launch_solve_stops_like_the_launched_cg(res):
+    bx, by, bz, b, _ = scenes.solve_problem(res, seed=35)
+    g = MGPCG(res, DEV, pre=2, post=2)
+    g.build_hierarchy(dev(bx), dev(by), dev(bz))
+    for rhs, max_iter in ((np.zeros_like(b), 10), (b, 0), (b, 1), (b, 4)):
+        (i1, r1, x1), (i2, r2, x2) = solves(g, res, rhs, 1e-30, max_iter)
+        assert i1 == i2 and abs(r1 - r2) <= 1e-4 * r2, (max_iter, r1, r2)
+        # the iterates of the two paths part by rounding
+        assert np.abs(x1 - x2).max() <= 1e-4 * max(np.abs(x2).max(), 1e-30)
+    bad = b.copy()
+    bad[1, 2, 3] = np.nan
+    with pytest.warns(RuntimeWarning):
+        g.solve(dev(bad), DeviceArray.zeros(res, device=DEV))
