@@ -248,11 +248,13 @@ __device__ __forceinline__ void p2g_grid(const P2GArgs& a, float* acc, int i, in
   box.flush(acc + a1 * PG_BOX, acc + a2 * PG_BOX, li, lj, lane);
 }
 
-__global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __grid_constant__ P2GArgs a) {
+// FACES = false: the cell grid alone (its two boxes come first in shared memory)
+template <bool FACES> __global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __grid_constant__ P2GArgs a) {
   extern __shared__ __align__(16) float acc[];  // [PG_NACC][PG_BOX]
+  constexpr int NACC = FACES ? PG_NACC : 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k0 = blockIdx.x * PG_TK, j0 = blockIdx.y * PG_TJ, i0 = blockIdx.z * PG_TI;
-  for (int e = tid; e < PG_NACC * PG_BOX; e += PG_NT) acc[e] = 0.f;
+  for (int e = tid; e < NACC * PG_BOX; e += PG_NT) acc[e] = 0.f;
   __syncthreads();
 
   const int nx = a.nx, ny = a.ny, nz = a.nz;
@@ -266,17 +268,19 @@ __global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __grid_constant__ P2GArg
       s = a.cell_start[key];
       e = a.cell_start[key + 1];
     }
-    p2g_grid<3>(a, acc, i, j, k, s, e, li, lj, lane);
-    p2g_grid<0>(a, acc, i, j, k, s, e, li, lj, lane);
-    p2g_grid<1>(a, acc, i, j, k, s, e, li, lj, lane);
-    p2g_grid<2>(a, acc, i, j, k, s, e, li, lj, lane);
+    p2g_grid<3>(a, FACES ? acc : acc - 6 * PG_BOX, i, j, k, s, e, li, lj, lane);
+    if (FACES) {
+      p2g_grid<0>(a, acc, i, j, k, s, e, li, lj, lane);
+      p2g_grid<1>(a, acc, i, j, k, s, e, li, lj, lane);
+      p2g_grid<2>(a, acc, i, j, k, s, e, li, lj, lane);
+    }
   }
   __syncthreads();
   // flush: each tile node once
-  for (int e = tid; e < PG_NACC * PG_BOX; e += PG_NT) {
+  for (int e = tid; e < NACC * PG_BOX; e += PG_NT) {
     const float v = acc[e];
     if (v == 0.f) continue;
-    const int arr = e / PG_BOX, b = e % PG_BOX;
+    const int arr = e / PG_BOX + (FACES ? 0 : 6), b = e % PG_BOX;
     const int g = arr < 6 ? arr % 3 : 3;
     const int li = b / (PG_BJ * PG_BK), lj = (b / PG_BK) % PG_BJ, lk = b % PG_BK;
     const int gi = i0 + li - (g == 0 ? 0 : 1);
@@ -295,8 +299,9 @@ using namespace pf;
 extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const float* vel4, const int32_t* cell_start,
                       float rho_l, float rho_g, float r_p, float* mass_x, float* mass_y, float* mass_z, float* mom_x,
                       float* mom_y, float* mom_z, float* cell_mass, float* cell_wsum, void* stream) {
-  PF_REQUIRE(g && pos4 && vel4 && cell_start && mass_x && mass_y && mass_z && mom_x && mom_y && mom_z && cell_mass &&
-                 cell_wsum,
+  const bool faces = mass_x || mass_y || mass_z || mom_x || mom_y || mom_z;
+  PF_REQUIRE(g && pos4 && vel4 && cell_start && cell_mass && cell_wsum &&
+                 (!faces || (mass_x && mass_y && mass_z && mom_x && mom_y && mom_z)),
              "null argument");
   PF_REQUIRE(g->nx > 0 && g->ny > 0 && g->nz > 0 && g->dx > 0.f, "bad grid");
   // the register boxes cover nodes within one cell of the particle's cell: the
@@ -305,11 +310,11 @@ extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const floa
   PF_REQUIRE(aligned16(pos4) && aligned16(vel4), "particle streams must be 16-byte aligned");
   static bool attr_set = false;
   if (!attr_set) {
-    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM));
+    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM));
     // the smallest shared-memory carveout that holds two CTAs' accumulators,
     // so that the rest of the SM's unified memory serves as L1 for the passes'
     // re-reads (a hint: the driver rounds up to a carveout it supports)
-    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g, cudaFuncAttributePreferredSharedMemoryCarveout, 40));
+    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 40));
     attr_set = true;
   }
   cudaStream_t s = S(stream);
@@ -318,7 +323,7 @@ extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const floa
                nc = (size_t)nx * ny * nz;
   float* outs[PG_NACC] = {mass_x, mass_y, mass_z, mom_x, mom_y, mom_z, cell_mass, cell_wsum};
   const size_t sizes[PG_NACC] = {fx, fy, fz, fx, fy, fz, nc, nc};
-  for (int q = 0; q < PG_NACC; ++q) PF_CUDA_TRY(cudaMemsetAsync(outs[q], 0, sizes[q] * sizeof(float), s));
+  for (int q = faces ? 0 : 6; q < PG_NACC; ++q) PF_CUDA_TRY(cudaMemsetAsync(outs[q], 0, sizes[q] * sizeof(float), s));
   if (n <= 0) return PF_OK;
   P2GArgs a;
   a.nx = nx; a.ny = ny; a.nz = nz;
@@ -331,7 +336,8 @@ extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const floa
   a.cell_start = cell_start;
   for (int q = 0; q < PG_NACC; ++q) a.out[q] = outs[q];
   dim3 grid((nz + PG_TK - 1) / PG_TK, (ny + PG_TJ - 1) / PG_TJ, (nx + PG_TI - 1) / PG_TI);
-  k_p2g<<<grid, PG_NT, PG_SMEM, s>>>(a);
+  if (faces) k_p2g<true><<<grid, PG_NT, PG_SMEM, s>>>(a);
+  else k_p2g<false><<<grid, PG_NT, PG_SMEM / PG_NACC * 2, s>>>(a);
   PF_LAUNCHED();
   return PF_OK;
 }

@@ -126,6 +126,8 @@ SIGNATURES = {
     "pf_adj_face_sources": (C.c_int, [_G] + [_VP] * 11 + [_VP] + [_F] * 7 + [_VP] * 15 + [_VP]),
     "pf_adj_p2g": (C.c_int, [_G, _I64, _VP, _VP, _F, _F, _F] + [_VP] * 7 + [_VP, _VP, _VP]),
     "pf_adj_phase_cell": (C.c_int, [_G, _VP, _VP, _F, _F, _F, _VP, _VP]),
+    "pf_phase_cell": (C.c_int, [_G, _VP, _F, _F, _F, _VP, _VP]),
+    "pf_adj_phase_particles": (C.c_int, [_G, _I64, _VP, _VP, _F, _F, _F, _VP, _VP, _VP]),
     "pf_adj_unsort": (C.c_int, [_I64, _VP, _VP, _VP, _VP, _VP, _VP]),
 }
 

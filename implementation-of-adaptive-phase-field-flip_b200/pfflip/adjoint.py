@@ -76,7 +76,6 @@ class DiffSim:
         self._lv_tmp = [torch.empty(s, dtype=torch.uint8, device=dev) for s in fs]
         self._gp = z(self.sim.res)
         self._lam = z(self.sim.res)
-        self._gphi_cell = z(self.sim.res)
         self._g4 = [torch.zeros((self.n, 4), dtype=torch.float32, device=dev) for _ in range(4)]
         self.adjoint_solves = []  # (iterations, residual) of every adjoint solve
 
@@ -215,28 +214,27 @@ class DiffSim:
         return _Phase.apply(x, self)
 
     def _phase_forward(self, x):
-        s = self.sim
-        self._load(x, torch.zeros_like(x))
-        s._p2g()
-        s._phase_field_and_coefficients()
-        return as_tensor(s.phi_cell).clone()
-
-    def _phase_backward(self, x, gphi):
+        """phi of the particles at x, and what its gradient needs: the sorted
+        particles, their places in the caller's order and the cell mass."""
         s, cfg = self.sim, self.cfg
         self._load(x, torch.zeros_like(x))
-        s._p2g()
-        s._phase_field_and_coefficients()
-        self._gphi_cell.copy_(gphi)
-        gcell = self._gp  # cell-sized scratch
-        N.call("pf_adj_phase_cell", C.byref(s._g), N.ptr(s.cell_mass), self._gphi_cell.data_ptr(),
-               float(s.rho_min), float(cfg.alpha_phi), float(s.rho_0l), gcell.data_ptr(), N.stream())
-        ga, gb = self._g4[0], self._g4[1]
-        ga.zero_()
-        gb.zero_()
-        N.call("pf_adj_p2g", C.byref(s._g), self.n, s._pos4.data_ptr(), s._vel4.data_ptr(), float(cfg.rho_l),
-               float(cfg.rho_g), float(np.float32(cfg.r_p)), None, None, None, None, None, None, gcell.data_ptr(),
-               ga.data_ptr(), gb.data_ptr(), N.stream())
-        return self._to_ids(ga)
+        # the cell grid alone: phi depends on nothing else
+        N.call("pf_p2g", C.byref(s._g), self.n, N.sptr(s._pos4), N.sptr(s._vel4), s._cell_start.data_ptr(),
+               float(cfg.rho_l), float(cfg.rho_g), float(np.float32(cfg.r_p)), *(None,) * 6, N.ptr(s.cell_mass),
+               N.ptr(s.cell_wsum), N.stream())
+        N.call("pf_phase_cell", C.byref(s._g), N.ptr(s.cell_mass), float(s.rho_min), float(cfg.alpha_phi),
+               float(s.rho_0l), N.ptr(s.phi_cell), N.stream())
+        return as_tensor(s.phi_cell).clone(), s._pos4.clone(), s._ids().clone(), as_tensor(s.cell_mass).clone()
+
+    def _phase_backward(self, pos4, ids, cell_mass, gphi):
+        s, cfg = self.sim, self.cfg
+        gcell = torch.empty_like(cell_mass)
+        N.call("pf_adj_phase_cell", C.byref(s._g), cell_mass.data_ptr(), gphi.data_ptr(), float(s.rho_min),
+               float(cfg.alpha_phi), float(s.rho_0l), gcell.data_ptr(), N.stream())
+        gx = torch.empty((self.n, 3), dtype=torch.float32, device=s.dev)
+        N.call("pf_adj_phase_particles", C.byref(s._g), self.n, N.sptr(pos4), N.sptr(ids), float(cfg.rho_l),
+               float(cfg.rho_g), float(np.float32(cfg.r_p)), gcell.data_ptr(), N.sptr(gx), N.stream())
+        return gx
 
 
 class _Block(torch.autograd.Function):
@@ -260,15 +258,15 @@ class _Phase(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, dsim):
         ctx.dsim = dsim
-        ctx.save_for_backward(x.detach().clone())
         with torch.no_grad():
-            return dsim._phase_forward(x)
+            phi, *saved = dsim._phase_forward(x.detach())
+        ctx.save_for_backward(*saved)
+        return phi
 
     @staticmethod
     def backward(ctx, gphi):
-        (x,) = ctx.saved_tensors
         with torch.no_grad():
-            gx = ctx.dsim._phase_backward(x, gphi.contiguous())
+            gx = ctx.dsim._phase_backward(*ctx.saved_tensors, gphi.to(torch.float32).contiguous())
         return gx, None
 
 

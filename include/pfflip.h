@@ -121,7 +121,8 @@ int pf_sort_particles_static(const pf_grid* g, int64_t n, const float* pos4_in, 
  * (p2g_cell) as launched by pfflip/sim.py:205-228, including the zeroing of the
  * 8 accumulators.  Eq. (6) weights with support radius r_p; particle mass is
  * rho_l for liquid, rho_g for air; particles with pstate != 0 are skipped.
- * Requires cell_start of the sort above (pos4/vel4 in sorted order). */
+ * Requires cell_start of the sort above (pos4/vel4 in sorted order).  With the
+ * six face arrays NULL only cell_mass and cell_wsum are formed. */
 int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const float* vel4, const int32_t* cell_start, float rho_l,
            float rho_g, float r_p, float* mass_x, float* mass_y, float* mass_z, float* mom_x, float* mom_y,
            float* mom_z, float* cell_mass, float* cell_wsum, void* stream);
@@ -446,6 +447,15 @@ int pf_adj_p2g(const pf_grid* g, int64_t n, const float* pos4, const float* vel4
  * zero on the clamped pieces. */
 int pf_adj_phase_cell(const pf_grid* g, const float* cell_mass, const float* gphi, float rho_min, float alpha_phi,
                       float rho_0l, float* gcell_mass, void* stream);
+
+/* eq. (7) on cells alone: phi_cell from cell_mass (pf_p2g with NULL face arrays),
+ * and the gradient of a loss on it in the particle positions: gpos[ids[t]] (rows
+ * of 3) from gcell_mass at the sorted position t; zero for droplets and dead
+ * particles. */
+int pf_phase_cell(const pf_grid* g, const float* cell_mass, float rho_min, float alpha_phi, float rho_0l,
+                  float* phi_cell, void* stream);
+int pf_adj_phase_particles(const pf_grid* g, int64_t n, const float* pos4, const int32_t* ids, float rho_l,
+                           float rho_g, float r_p, const float* gcell_mass, float* gpos, void* stream);
 
 /* Adjoint of the sort's gather: out[perm[t]] = in[t] for both streams. */
 int pf_adj_unsort(int64_t n, const int32_t* perm, const float* gpos4_sorted, const float* gvel4_sorted,

@@ -49,3 +49,38 @@ def test_particles_round_trip(n, kind):
         assert (po is None or x is po) and (vo is None or v is vo)
         torch.cuda.synchronize()
         assert np.array_equal(x.cpu().numpy(), pos) and np.array_equal(v.cpu().numpy(), vel)
+
+
+@pytest.mark.parametrize("res,ppc", [((6, 5, 4), 8), ((16, 16, 16), 8), ((33, 9, 12), 27)])
+def test_phase_field_and_gradient_match_the_step_kernels(res, ppc):
+    """phase_field forms the cell grid alone and its gradient in one pass: equal
+    to the step's stages (same sums) and, for the gradient, to the general
+    adjoint gather within the rounding of eight products, 1e-5 of the maximum."""
+    import ctypes as C
+
+    from pfflip import _native as N
+    from pfflip import scenes
+    from pfflip.adjoint import DiffSim
+
+    cfg = Config(res=res, dx=1.0 / max(res), ppc=ppc, droplets=False, device=DEV)
+    pos, _, typ = scenes.dam_break(cfg)
+    ds = DiffSim(cfg, typ, 1e-3)
+    x = torch.from_numpy(pos).to(DEV).requires_grad_(True)
+    phi = ds.phase_field(x)
+    w = torch.randn(res, device=DEV, generator=torch.Generator(DEV).manual_seed(1))
+    (gx,) = torch.autograd.grad(phi, x, w)
+    s = ds.sim
+    s.set_particles(pos, np.zeros_like(pos), typ)
+    s._p2g()
+    s._phase_field_and_coefficients()
+    assert np.abs(s.phi_cell.numpy() - phi.detach().cpu().numpy()).max() < 1e-5
+    gcell = torch.empty_like(w)
+    N.call("pf_adj_phase_cell", C.byref(s._g), N.ptr(s.cell_mass), w.data_ptr(), float(s.rho_min), float(cfg.alpha_phi),
+           float(s.rho_0l), gcell.data_ptr(), N.stream())
+    ga, gb = (torch.zeros(len(pos), 4, device=DEV) for _ in range(2))
+    N.call("pf_adj_p2g", C.byref(s._g), len(pos), s._pos4.data_ptr(), s._vel4.data_ptr(), float(cfg.rho_l),
+           float(cfg.rho_g), float(np.float32(cfg.r_p)), *(None,) * 6, gcell.data_ptr(), ga.data_ptr(), gb.data_ptr(),
+           N.stream())
+    ref = torch.empty(len(pos), 3, device=DEV)
+    ref[s._ids().long()] = ga[:, :3]
+    assert (ref - gx).abs().max() <= 1e-5 * ref.abs().max()
