@@ -210,8 +210,8 @@ template <int G> struct Box {
 
 // one grid over the particles of cell (i, j, k) (range [s, e)), then the row flush
 template <int G>
-__device__ __forceinline__ void p2g_grid(const P2GArgs& a, float* acc, int i, int j, int k, int s, int e, int li,
-                                         int lj, int lane) {
+__device__ __forceinline__ void p2g_grid(const P2GArgs& a, float* sm1, float* sm2, int i, int j, int k, int s, int e,
+                                         int li, int lj, int lane) {
   Box<G> box;
   box.zero();
   const float ci = (float)i, cj = (float)j, ck = (float)k;
@@ -244,16 +244,26 @@ __device__ __forceinline__ void p2g_grid(const P2GArgs& a, float* acc, int i, in
                         fmaf(ck, -a.dx, P.z) * a.inv_r};
     box.add(X, mp, up, a.s_node);
   }
-  const int a1 = (G < 3) ? G : 6, a2 = (G < 3) ? 3 + G : 7;
-  box.flush(acc + a1 * PG_BOX, acc + a2 * PG_BOX, li, lj, lane);
+  box.flush(sm1, sm2, li, lj, lane);
 }
 
-// FACES = false: the cell grid alone (its two boxes come first in shared memory)
-template <bool FACES> __global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __grid_constant__ P2GArgs a) {
-  extern __shared__ __align__(16) float acc[];  // [PG_NACC][PG_BOX]
-  constexpr int NACC = FACES ? PG_NACC : 2;
+// MODE ALL: a warp passes over its row once per grid, so three of the four
+// passes find the row's particles in L1.  CELLS: the cell grid alone.  SPLIT: one
+// grid per CTA, blockIdx.z counting the tiles of one grid after another (so CTAs
+// that run together run the same code): four times the warps, and an 11 KB
+// accumulator that leaves room for three CTAs per SM, for four reads of the
+// particles.  MINB: CTAs per SM the registers are held to (three spill 148
+// bytes, which pays only where there are CTAs to fill them).
+enum { P2G_ALL, P2G_CELLS, P2G_SPLIT };
+
+template <int MODE, int MINB>
+__global__ void __launch_bounds__(PG_NT, MINB) k_p2g(const __grid_constant__ P2GArgs a) {
+  extern __shared__ __align__(16) float acc[];  // accumulator boxes in the order of a.out
+  constexpr int NACC = MODE == P2G_ALL ? PG_NACC : 2;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int k0 = blockIdx.x * PG_TK, j0 = blockIdx.y * PG_TJ, i0 = blockIdx.z * PG_TI;
+  const int tiles_i = (a.nx + PG_TI - 1) / PG_TI;
+  const int split = MODE == P2G_SPLIT ? (int)blockIdx.z / tiles_i : 0;  // 0: cells, then the faces
+  const int k0 = blockIdx.x * PG_TK, j0 = blockIdx.y * PG_TJ, i0 = ((int)blockIdx.z - split * tiles_i) * PG_TI;
   for (int e = tid; e < NACC * PG_BOX; e += PG_NT) acc[e] = 0.f;
   __syncthreads();
 
@@ -268,11 +278,16 @@ template <bool FACES> __global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __
       s = a.cell_start[key];
       e = a.cell_start[key + 1];
     }
-    p2g_grid<3>(a, FACES ? acc : acc - 6 * PG_BOX, i, j, k, s, e, li, lj, lane);
-    if (FACES) {
-      p2g_grid<0>(a, acc, i, j, k, s, e, li, lj, lane);
-      p2g_grid<1>(a, acc, i, j, k, s, e, li, lj, lane);
-      p2g_grid<2>(a, acc, i, j, k, s, e, li, lj, lane);
+    if constexpr (MODE == P2G_ALL) {
+      p2g_grid<3>(a, acc + 6 * PG_BOX, acc + 7 * PG_BOX, i, j, k, s, e, li, lj, lane);
+      p2g_grid<0>(a, acc, acc + 3 * PG_BOX, i, j, k, s, e, li, lj, lane);
+      p2g_grid<1>(a, acc + PG_BOX, acc + 4 * PG_BOX, i, j, k, s, e, li, lj, lane);
+      p2g_grid<2>(a, acc + 2 * PG_BOX, acc + 5 * PG_BOX, i, j, k, s, e, li, lj, lane);
+    } else {
+      if (MODE == P2G_CELLS || split == 0) p2g_grid<3>(a, acc, acc + PG_BOX, i, j, k, s, e, li, lj, lane);
+      else if (split == 1) p2g_grid<0>(a, acc, acc + PG_BOX, i, j, k, s, e, li, lj, lane);
+      else if (split == 2) p2g_grid<1>(a, acc, acc + PG_BOX, i, j, k, s, e, li, lj, lane);
+      else p2g_grid<2>(a, acc, acc + PG_BOX, i, j, k, s, e, li, lj, lane);
     }
   }
   __syncthreads();
@@ -280,7 +295,8 @@ template <bool FACES> __global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __
   for (int e = tid; e < NACC * PG_BOX; e += PG_NT) {
     const float v = acc[e];
     if (v == 0.f) continue;
-    const int arr = e / PG_BOX + (FACES ? 0 : 6), b = e % PG_BOX;
+    const int q = e / PG_BOX, b = e % PG_BOX;
+    const int arr = MODE == P2G_ALL ? q : split == 0 ? 6 + q : split - 1 + 3 * q;
     const int g = arr < 6 ? arr % 3 : 3;
     const int li = b / (PG_BJ * PG_BK), lj = (b / PG_BK) % PG_BJ, lk = b % PG_BK;
     const int gi = i0 + li - (g == 0 ? 0 : 1);
@@ -290,6 +306,22 @@ template <bool FACES> __global__ void __launch_bounds__(PG_NT, 2) k_p2g(const __
     if (gi < 0 || gj < 0 || gk < 0 || gi >= n0 || gj >= n1 || gk >= n2) continue;
     atomicAdd(a.out[arr] + ((long long)gi * n1 + gj) * n2 + gk, v);
   }
+}
+
+// the accumulators zeroed in one launch (blockIdx.y: array); 16 bytes a store
+// where the array starts on a 16-byte boundary
+struct P2GZero {
+  float* p[PG_NACC];
+  long long n[PG_NACC];
+};
+
+__global__ void __launch_bounds__(256) k_p2g_zero(const __grid_constant__ P2GZero z) {
+  float* p = z.p[blockIdx.y];
+  if (!p) return;
+  const long long n = z.n[blockIdx.y], t0 = (long long)blockIdx.x * 256 + threadIdx.x, step = (long long)gridDim.x * 256;
+  const long long n4 = (reinterpret_cast<uintptr_t>(p) & 15u) == 0 ? n >> 2 : 0;
+  for (long long e = t0; e < n4; e += step) reinterpret_cast<float4*>(p)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (long long e = 4 * n4 + t0; e < n; e += step) p[e] = 0.f;
 }
 
 }  // namespace pf
@@ -310,11 +342,11 @@ extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const floa
   PF_REQUIRE(aligned16(pos4) && aligned16(vel4), "particle streams must be 16-byte aligned");
   static bool attr_set = false;
   if (!attr_set) {
-    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM));
+    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g<P2G_ALL, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM));
     // the smallest shared-memory carveout that holds two CTAs' accumulators,
     // so that the rest of the SM's unified memory serves as L1 for the passes'
     // re-reads (a hint: the driver rounds up to a carveout it supports)
-    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g<true>, cudaFuncAttributePreferredSharedMemoryCarveout, 40));
+    PF_CUDA_TRY(cudaFuncSetAttribute(k_p2g<P2G_ALL, 2>, cudaFuncAttributePreferredSharedMemoryCarveout, 40));
     attr_set = true;
   }
   cudaStream_t s = S(stream);
@@ -323,7 +355,13 @@ extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const floa
                nc = (size_t)nx * ny * nz;
   float* outs[PG_NACC] = {mass_x, mass_y, mass_z, mom_x, mom_y, mom_z, cell_mass, cell_wsum};
   const size_t sizes[PG_NACC] = {fx, fy, fz, fx, fy, fz, nc, nc};
-  for (int q = faces ? 0 : 6; q < PG_NACC; ++q) PF_CUDA_TRY(cudaMemsetAsync(outs[q], 0, sizes[q] * sizeof(float), s));
+  P2GZero z;
+  for (int q = 0; q < PG_NACC; ++q) {
+    z.p[q] = faces || q >= 6 ? outs[q] : nullptr;
+    z.n[q] = (long long)sizes[q];
+  }
+  k_p2g_zero<<<dim3(grid_for((long long)(fx / 4), 256, kNumSMs * 2), PG_NACC), 256, 0, s>>>(z);
+  PF_LAUNCHED();
   if (n <= 0) return PF_OK;
   P2GArgs a;
   a.nx = nx; a.ny = ny; a.nz = nz;
@@ -336,8 +374,20 @@ extern "C" int pf_p2g(const pf_grid* g, int64_t n, const float* pos4, const floa
   a.cell_start = cell_start;
   for (int q = 0; q < PG_NACC; ++q) a.out[q] = outs[q];
   dim3 grid((nz + PG_TK - 1) / PG_TK, (ny + PG_TJ - 1) / PG_TJ, (nx + PG_TI - 1) / PG_TI);
-  if (faces) k_p2g<true><<<grid, PG_NT, PG_SMEM, s>>>(a);
-  else k_p2g<false><<<grid, PG_NT, PG_SMEM / PG_NACC * 2, s>>>(a);
+  const size_t box2 = PG_SMEM / PG_NACC * 2;
+  const dim3 grid4(grid.x, grid.y, 4 * grid.z);
+  // Few tiles: the split, whose four times as many CTAs run at once (us with the
+  // zeroing, split against all: 16^3 / 8 particles per cell 43, 76; 32^3 / 27 68,
+  // 123; 48^3 / 8 103, 113).  Enough tiles for two CTAs on every SM: the split
+  // where cells hold few particles, so that a pass is mostly the latency of its
+  // first loads and its box flush (64^3 / 8 158, 182; 128^3 / 8 1007, 1176; 256^3
+  // / 8 7755, 8530); the row passes where they hold many and the re-reads count
+  // (64^3 / 27 360, 344; 128^3 / 27 2495, 2128).  The line at 16 lies between.
+  const long long tiles = (long long)grid.x * grid.y * grid.z, cells = (long long)nx * ny * nz;
+  if (!faces) k_p2g<P2G_CELLS, 2><<<grid, PG_NT, box2, s>>>(a);
+  else if (tiles < 2 * kNumSMs && 4 * grid.z <= 65535) k_p2g<P2G_SPLIT, 2><<<grid4, PG_NT, box2, s>>>(a);
+  else if (n < 16 * cells && 4 * grid.z <= 65535) k_p2g<P2G_SPLIT, 3><<<grid4, PG_NT, box2, s>>>(a);
+  else k_p2g<P2G_ALL, 2><<<grid, PG_NT, PG_SMEM, s>>>(a);
   PF_LAUNCHED();
   return PF_OK;
 }
