@@ -151,25 +151,27 @@ class DiffSim:
             self.sim.step(self.dt)
         return self._to_ids(self.sim._pos4), self._to_ids(self.sim._vel4)
 
-    def _saved_fields(self):
+    def _field_arrays(self):
         s = self.sim
-        return [as_tensor(a) for a in (*s.vel, *s.vel_star, *s.vel_liq, *s.beta, *s.mass, *s.mom, s.is_liquid,
-                                        s.pressure)]
+        return (*s.vel, *s.vel_star, *s.vel_liq, *s.beta, *s.mass, *s.mom, s.is_liquid, s.pressure)
 
-    def _snapshot(self):
-        """Everything the step's adjoint reads, right after its grid stages: the
-        sorted particles, the sort permutation and the grid fields."""
+    def _take_fields(self):
+        """The sort permutation and the grid fields of the step just run, handed
+        over as they are: the simulator goes on with fresh arrays, of which its
+        next step writes every element."""
         s = self.sim
-        return (s._pos4.clone(), s._vel4.clone(), s._perm.clone(), [t.clone() for t in self._saved_fields()])
+        perm, s._perm = s._perm, torch.empty_like(s._perm)
+        fields = [a.tensor for a in self._field_arrays()]
+        for a in self._field_arrays():
+            a.tensor = torch.empty_like(a.tensor)
+        return perm, fields
 
-    def _restore(self, snap):
+    def _give_back(self, snap):
+        """Make a step's state, as its grid stages left it, the simulator's."""
         s = self.sim
-        p4, v4, perm, fields = snap
-        s._pos4.copy_(p4)
-        s._vel4.copy_(v4)
-        s._perm.copy_(perm)
-        for t, src in zip(self._saved_fields(), fields):
-            t.copy_(src)
+        s._pos4, s._vel4, (s._perm, fields) = snap
+        for a, t in zip(self._field_arrays(), fields):
+            a.tensor = t
         s.solver.build_hierarchy(*s.beta)  # the adjoint solve uses this step's operator
         s._particles_changed()
 
@@ -182,15 +184,17 @@ class DiffSim:
         self._load(x, v)
         s._particles_changed()  # step 0 sorts again (the identity), so its permutation maps onto this order
         snaps = []
-        for _ in range(nsteps):
+        for k in range(nsteps):
             self._grid_stages()
-            snaps.append(self._snapshot())
-            s._g2p_advect(self.dt, do_g2p=True, do_advect=True)
+            if k < nsteps - 1:  # the last step's state is used where it stands
+                p4, v4 = s._pos4.clone(), s._vel4.clone()
+                s._g2p_advect(self.dt, do_g2p=True, do_advect=True)
+                snaps.append((p4, v4, self._take_fields()))
         ga, gb = self._g4[0], self._g4[1]
         self._from_ids(gx, gv, ga, gb)
         for k in range(nsteps - 1, -1, -1):
-            self._restore(snaps[k])
-            snaps[k] = None
+            if k < nsteps - 1:
+                self._give_back(snaps.pop())
             # ga/gb are in the order of the arrays after the step, which is the
             # order after the step's sort; the result is in the order before it
             nxt_p, nxt_v = torch.empty_like(ga), torch.empty_like(gb)
