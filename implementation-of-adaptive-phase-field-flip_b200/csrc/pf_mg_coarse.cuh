@@ -453,10 +453,12 @@ template <class T, int NQ> struct CoarseCycle {
   }
 
   // end of a step on the level at hand after `n` exchanges: its CTAs see the
-  // new values.  A neighbour's next store into a halo plane cannot overtake
-  // this CTA's reads of it: it waits for the stores of exactly the threads
-  // that read that plane, and its store after next (the same barrier again)
-  // for this CTA's next exchange.
+  // new values.  With a settle after every exchange, a neighbour's next store
+  // into a halo plane cannot overtake this CTA's reads of it: it waits for the
+  // stores of exactly the threads that read that plane.  Nor can its store after
+  // next, on the same barrier and of the same colour, overtake this one: it
+  // waits for this CTA's next exchange, which follows this settle.  Two
+  // exchanges before one settle need a cluster barrier before the next exchange.
   __device__ __forceinline__ void settle(int n) {
     if (s == 0) return;
     __syncthreads();
@@ -592,9 +594,11 @@ template <class T, int NQ> struct CoarseCycle {
       v0[u] = f2_fma(v, sc, p[0][u]);
       v1[u] = f2_fma(v, sc, p[1][u]);
     }
+    // one exchange, of colour 0: the post-sweeps begin with colour 1, which reads
+    // colour 0 and then sends its own
     put<0>(v0, true);
-    put<1>(v1, true);
-    settle(2);
+    put<1>(v1, false);
+    settle(1);
   }
 
   // sum over the CTAs of level l of a per-thread value, in every thread of them
@@ -843,7 +847,7 @@ template <class T, int NQ> struct CoarseCycle {
         }
       }
       if (s > 0) prolong(l);
-      else turn += 2u;
+      else ++turn;
       if (l == 0) cc_arrive();  // done with the other CTAs' shared memory
       sweeps(a.post, 1, false);
     }
