@@ -601,7 +601,10 @@ template <class T, int NQ> struct CoarseCycle {
     settle(1);
   }
 
-  // sum over the CTAs of level l of a per-thread value, in every thread of them
+  // sum over the CTAs of level l of a per-thread value, in every thread of them.
+  // A CTA reads its s_part after the cluster barrier in here, so the next sum into
+  // the same s_part needs another cluster barrier before it; sums without one take
+  // another s_part.
   __device__ __forceinline__ double level_sum(int l, double v, double* sred, double* s_part) {
     const CcLevel& L = a.L[l];
     v = block_sum<CC_NT>(v, sred);
@@ -860,7 +863,7 @@ template <class T, int NQ>
 __global__ void __launch_bounds__(CC_NT, 1) k_coarse(const __grid_constant__ CcArgs a) {
   extern __shared__ __align__(16) float ccsm[];
   __shared__ double sred[40];
-  __shared__ double s_part[CC_MAXC + 1];
+  __shared__ double s_part[CC_MAXC + 1], s_mean[CC_MAXC + 1];
   CoarseCycle<T, NQ> cy(a, ccsm);
   cy.stage_dense();
   cy.init_barriers();
@@ -898,7 +901,7 @@ __global__ void __launch_bounds__(CC_NT, 1) k_coarse(const __grid_constant__ CcA
     }
   }
   if (a.want_mean) {
-    const double tot = cy.level_sum(0, ls, sred, s_part);
+    const double tot = cy.level_sum(0, ls, sred, s_mean);
     if (cy.rank == L.c0 && cy.tid == 0) {
       const double n = (double)L.n0 * L.n1 * L.n2;
       a.st->sum_last = tot;

@@ -166,12 +166,20 @@ class DiffSim:
             a.tensor = torch.empty_like(a.tensor)
         return perm, fields
 
+    def _own(self, perm, fields):
+        self.sim._perm = perm
+        for a, t in zip(self._field_arrays(), fields):
+            a.tensor = t
+
     def _give_back(self, snap):
         """Make a step's state, as its grid stages left it, the simulator's."""
         s = self.sim
-        s._pos4, s._vel4, (s._perm, fields) = snap
-        for a, t in zip(self._field_arrays(), fields):
-            a.tensor = t
+        p4, v4, taken = snap
+        # copied back: the simulator's own streams may have been allocated on
+        # another stream than this pass's, so they are neither dropped nor replaced
+        s._pos4.copy_(p4)
+        s._vel4.copy_(v4)
+        self._own(*taken)
         s.solver.build_hierarchy(*s.beta)  # the adjoint solve uses this step's operator
         s._particles_changed()
 
@@ -182,6 +190,14 @@ class DiffSim:
         step's adjoint instead of recomputing the step's grid stages."""
         s = self.sim
         self._load(x, v)
+        own = s._perm, [a.tensor for a in self._field_arrays()]
+        try:
+            return self._replay_and_walk_back(nsteps, gx, gv)
+        finally:  # the arrays the simulator was made with are its own again, after an error too
+            self._own(*own)
+
+    def _replay_and_walk_back(self, nsteps, gx, gv):
+        s = self.sim
         s._particles_changed()  # step 0 sorts again (the identity), so its permutation maps onto this order
         snaps = []
         for k in range(nsteps):
@@ -263,14 +279,21 @@ class _Phase(torch.autograd.Function):
     def forward(ctx, x, dsim):
         ctx.dsim = dsim
         with torch.no_grad():
-            phi, *saved = dsim._phase_forward(x.detach())
-        ctx.save_for_backward(*saved)
+            phi, pos4, ids, cell_mass = dsim._phase_forward(x.detach())
+        # the streams hold integers in their words, which a saved-tensor hook may
+        # not keep (and the kernel writes to the places that ids names), so only
+        # the mass is saved as autograd saves
+        ctx.particles = pos4, ids
+        ctx.save_for_backward(cell_mass)
         return phi
 
     @staticmethod
     def backward(ctx, gphi):
+        (mass,) = ctx.saved_tensors
+        dev = ctx.dsim.sim.dev
         with torch.no_grad():
-            gx = ctx.dsim._phase_backward(*ctx.saved_tensors, gphi.to(torch.float32).contiguous())
+            mass, gphi = (t.to(device=dev, dtype=torch.float32).contiguous() for t in (mass, gphi))
+            gx = ctx.dsim._phase_backward(*ctx.particles, mass, gphi)
         return gx, None
 
 

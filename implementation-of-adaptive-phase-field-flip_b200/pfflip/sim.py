@@ -283,13 +283,21 @@ class Simulator:
         pending = []
         n = self.n_particles
 
-        def direct(d):  # a device tensor that takes the rows as they are
+        def direct(d):
+            # a device tensor that takes the rows as they are.  The copy below is
+            # for what only torch can write or refuse to: tensors that take part
+            # in autograd, in reverse or forward mode, and inference tensors
             return (d is not None and d.device == self.dev and d.dtype == torch.float32 and d.is_contiguous()
-                    and d.shape == (n, 3))
+                    and d.shape == (n, 3) and not d.requires_grad and not d.is_inference()
+                    and torch.autograd.forward_ad.unpack_dual(d).tangent is None)
 
-        if direct(pos_out) and direct(vel_out):
+        def apart(a, b):  # the velocities are written over positions in the same memory, not beside them
+            return abs(a.data_ptr() - b.data_ptr()) >= 12 * n
+
+        if direct(pos_out) and direct(vel_out) and apart(pos_out, vel_out):
             N.call("pf_unpack_particles", n, N.sptr(self._vel4), N.sptr(self._pos4), N.ptr(pos_out),
                    N.sptr(self._vel4), N.ptr(vel_out), N.stream())
+            torch.autograd.graph.increment_version((pos_out, vel_out))  # as an in-place copy does
             self._pending_d2h = []
             return pos_out, vel_out
         for src, dst in ((self._pos4, pos_out), (self._vel4, vel_out)):

@@ -241,3 +241,40 @@ def test_rt_amplitude_gradient_matches_fp64_finite_differences():
         if len(checked) == 2:
             break
     assert len(checked) == 2, checked
+
+
+def test_backward_passes_leave_the_simulator_its_own_arrays():
+    """Two backward passes in a row give the same gradient, a step after them is
+    the step of a fresh simulator, and the simulator still holds the arrays it
+    was made with (they may belong to another stream than the backward pass's).
+    The gradients differ by the order of atomic sums: 1e-4 of the maximum through
+    three steps and their solves to 1e-6; the positions by 1e-5 of a cell's size."""
+    from pfflip import Simulator
+
+    cfg = small_cfg()
+    dt = step_dt(cfg)
+    pos, vel, ptype, _, _ = scenes.asteroid_pool(cfg)
+    ds = DiffSim(cfg, ptype, dt, checkpoint_every=3, adjoint_tol=1e-6)
+    x0 = torch.tensor(pos, device=DEV, requires_grad=True)
+    v0 = torch.tensor(vel, device=DEV, requires_grad=True)
+    w = torch.randn(len(pos), 3, device=DEV, generator=torch.Generator(DEV).manual_seed(5))
+    ds.sim.set_particles(x0.detach(), v0.detach(), ptype)  # the streams are allocated
+
+    def arrays():
+        s = ds.sim
+        return {t.data_ptr() for t in (s._pos4, s._pos4_alt, s._vel4, s._vel4_alt, s._perm,
+                                       *(a.tensor for a in ds._field_arrays()))}
+
+    own = arrays()
+    grads = []
+    for _ in range(2):
+        xT, vT = ds.rollout(x0, v0, 3)
+        grads.append(torch.autograd.grad((w * xT).sum() + (w * vT).sum(), (x0, v0)))
+        assert arrays() == own
+    for a, b in zip(*grads):
+        assert (a - b).abs().max() <= 1e-4 * a.abs().max()
+    fresh = Simulator(cfg)
+    for s in (ds.sim, fresh):
+        s.set_particles(pos, vel, ptype)
+        s.step(dt)
+    assert np.abs(ds.sim.px.numpy() - fresh.px.numpy()).max() <= 1e-5 * cfg.dx

@@ -1,5 +1,5 @@
-"""The halo exchange of the cluster kernels (csrc/pf_mg_coarse.cuh) under every
-order in which its warps and messages can run.
+"""The halo exchange and the sums of the cluster kernels (csrc/pf_mg_coarse.cuh)
+under every order in which warps and messages can run.
 
 The steps of a half-sweep, of the prolongation and of the CG's product are read
 from the source and run by a model of two neighbouring CTAs.  In each, one warp
@@ -156,6 +156,55 @@ def test_halo_exchange_in_every_order(name):
         s = todo.pop()
         nxt = list(moves(s))
         assert nxt or all(c[0] == c[1] == len(prog) for c in s), f"a wait that never ends at {s} of {prog}"
+        for n in nxt:
+            if n not in seen:
+                seen.add(n)
+                todo.append(n)
+
+
+def test_sums_in_a_row_in_every_order():
+    """The mean of a swept coarsest level and the mean of the result follow each
+    other with no cluster barrier between when that level is the only one.  A sum
+    writes the CTA's part into every CTA's buffer, passes the cluster barrier and
+    reads the buffer; a CTA whose reads are late must not find the next sum's
+    parts there."""
+    coarsest = re.findall(r"level_sum\(l, t, sred, (\w+)\)", body(r"void coarsest_solve\("))
+    kernel = body(r"\bk_coarse\(const")
+    (cycle,) = re.findall(r"cy\.cycle\(sred, (\w+)\)", kernel)
+    (last,) = re.findall(r"level_sum\(0, ls, sred, (\w+)\)", kernel)
+    assert coarsest and all(b == "s_part" for b in coarsest)  # the cycle's argument
+    bufs = [cycle, last]
+    prog = []
+    for k, b in enumerate(bufs):
+        prog += [("sync", k), ("write", k), ("cluster", k), ("read", k)]
+    # per CTA: pc of the warp that writes, pc of a warp that only reads; who wrote each (buffer, part) last
+    start = (((0, 0), (0, 0)), frozenset())
+    seen, todo = {start}, [start]
+    while todo:
+        pcs, mem = todo.pop()
+        found = dict(mem)
+        nxt = []
+        for c in range(2):
+            for w in range(2):
+                if pcs[c][w] == len(prog):
+                    continue
+                op, k = prog[pcs[c][w]]
+                one = tuple(tuple(pcs[a][b] + (a == c and b == w) for b in range(2)) for a in range(2))
+                if op == "write":
+                    new = dict(found)
+                    if w == 0:
+                        new[bufs[k], 0, c] = new[bufs[k], 1, c] = k  # part c in the buffers of both CTAs
+                    nxt.append((one, frozenset(new.items())))
+                elif op == "read":
+                    for part in range(2):
+                        assert found[bufs[k], c, part] == k, f"sum {k} read a part of sum {found[bufs[k], c, part]}"
+                    nxt.append((one, mem))
+                elif op == "sync" and w == 0 and pcs[c][0] == pcs[c][1]:
+                    both = tuple(tuple(pcs[a][b] + (a == c) for b in range(2)) for a in range(2))
+                    nxt.append((both, mem))
+                elif op == "cluster" and c == w == 0 and len({p for q in pcs for p in q}) == 1:
+                    nxt.append((tuple(tuple(p + 1 for p in q) for q in pcs), mem))
+        assert nxt or all(p == len(prog) for q in pcs for p in q)
         for n in nxt:
             if n not in seen:
                 seen.add(n)
