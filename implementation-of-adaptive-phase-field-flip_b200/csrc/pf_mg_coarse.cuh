@@ -951,9 +951,11 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
   __shared__ double s_warp[CC_RED][CC_NT / 32];
   __shared__ double s_all[2][CC_RED][CC_MAXC];
   __shared__ int s_go[2];
+  __shared__ int s_fail;  // in the top level's first CTA: a wait of some thread of the cluster ran out
   const CcArgs& a = A.cc;
   CoarseCycle<T, NQ> cy(a, ccsm);
   const int tid = cy.tid;
+  if (tid == 0) s_fail = 0;
   const CcLevel& L = a.L[0];
   cy.stage_dense();
   cy.init_barriers();
@@ -1194,7 +1196,7 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
         }
       cur ^= 1;
     }
-    red[0] = (double)m;
+    red[0] = cy.fail ? (double)INFINITY : (double)m;  // a wait that ran out ends the iteration everywhere
     reduce(k1, mx, red);
     if (go) {
       rel = red[0] / bnorm;
@@ -1234,15 +1236,17 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
     for (int d = 0; d < 4; ++d)
       if (4 * h + d < L.n2) out[row * L.n2 + 4 * h + d] = v[d] + cx;
   }
-  if (mine && cy.rank == L.c0 && tid == 0) {
+  if (cy.fail)
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cc_map(smem_u32(&s_fail), L.c0)), "r"(1) : "memory");
+  if (a.C > 1) cc_sync();  // no CTA leaves while another may still write to it
+  else __syncthreads();
+  if (cy.rank == L.c0 && tid == 0) {
     a.st->it = it;
     a.st->rel = rel;
     a.st->bnorm = bnorm;
-    a.st->status = status;
+    a.st->status = s_fail ? ST_TMA_TIMEOUT : status;
     a.st->done = 1;
   }
-  if (cy.fail) a.st->status = ST_TMA_TIMEOUT;
-  if (a.C > 1) cc_sync();  // no CTA leaves while another may still write to it
 }
 
 }  // namespace pf

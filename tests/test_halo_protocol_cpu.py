@@ -209,3 +209,18 @@ def test_sums_in_a_row_in_every_order():
             if n not in seen:
                 seen.add(n)
                 todo.append(n)
+
+
+def test_an_expired_wait_reaches_the_status_of_a_solve():
+    """The flag of a thread whose wait ran out goes to the CTA that stores the
+    status, before the cluster barrier after which that CTA stores it, and no
+    other thread stores a status.  It also ends the iteration: the value that all
+    CTAs compare with the tolerance becomes infinite."""
+    code = body(r"\bk_solve\(const")
+    stores = [m.start() for m in re.finditer(r"a\.st->status\s*=", code)]
+    assert len(stores) == 1
+    tail = code[:stores[0]]
+    flag, barrier = tail.rindex("smem_u32(&s_fail), L.c0)"), tail.rindex("cc_sync();")
+    assert flag < barrier and "s_fail ? ST_TMA_TIMEOUT : status" in code[stores[0]:]
+    loop = code[code.index("while (agree(go))"):barrier]
+    assert re.search(r"red\[0\] = cy\.fail \? \(double\)INFINITY[^;]*;\s*reduce\(k1, mx, red\)", loop)
