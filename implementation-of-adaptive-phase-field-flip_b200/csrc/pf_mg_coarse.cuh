@@ -15,7 +15,7 @@
 //   load, lanes on consecutive words), its neighbours along k are the thread's
 //   own registers and one more word.  Walls need no tests: their coefficients
 //   are zero and one halo plane on either side keeps every address inside.
-// * A level of more than CC_NT * 2 quads is split into slabs of planes over the
+// * A level of more than CC_NT * 2 quads (CC_NT * 3 for FP64 sweeps) is split into slabs of planes over the
 //   cluster's CTAs; a thread that relaxes a boundary plane also stores its pair
 //   into the neighbour's halo plane (st.async, counted on the neighbour's
 //   mbarrier), so a half-sweep waits for its two neighbours and not for the
@@ -40,7 +40,8 @@
 // 16-bit hierarchies: storage is widened on load, p stays FP32 inside the
 // kernel, the right-hand sides of the levels and the result are rounded to the
 // storage type; the coarsest solve (sweeps on one CTA, or the dense operator)
-// runs in FP64.
+// runs in FP64.  A swept coarsest level of more than 4096 cells, in slabs, is
+// swept in FP32.
 #pragma once
 
 #include "pf_f32x2.cuh"
