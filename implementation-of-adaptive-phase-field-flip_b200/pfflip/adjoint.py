@@ -279,14 +279,21 @@ class _Phase(torch.autograd.Function):
     def forward(ctx, x, dsim):
         ctx.dsim = dsim
         with torch.no_grad():
-            phi, *saved = dsim._phase_forward(x.detach())
-        ctx.save_for_backward(*saved)
+            phi, pos4, ids, cell_mass = dsim._phase_forward(x.detach())
+        # the streams hold integers in their words, which a saved-tensor hook may
+        # not keep (and the kernel writes to the places that ids names), so only
+        # the mass is saved as autograd saves
+        ctx.particles = pos4, ids
+        ctx.save_for_backward(cell_mass)
         return phi
 
     @staticmethod
     def backward(ctx, gphi):
+        (mass,) = ctx.saved_tensors
+        dev = ctx.dsim.sim.dev
         with torch.no_grad():
-            gx = ctx.dsim._phase_backward(*ctx.saved_tensors, gphi.to(torch.float32).contiguous())
+            mass, gphi = (t.to(device=dev, dtype=torch.float32).contiguous() for t in (mass, gphi))
+            gx = ctx.dsim._phase_backward(*ctx.particles, mass, gphi)
         return gx, None
 
 
