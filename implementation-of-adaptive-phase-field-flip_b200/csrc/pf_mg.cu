@@ -2740,6 +2740,10 @@ template <class T> int enqueue_whole(pf_mg_plan* P, const float* b, float* x, fl
   CcSolveArgs A = P->cs;
   A.cc = coarse_args<T, float>(P, b);
   A.x = x;
+  A.x_raw = P->d.x;
+  A.rhs = P->d.rhs;
+  A.res[0] = P->d.res_v;
+  A.res[1] = P->d.res_alt;
   A.tol = tol;
   A.max_iter = max_iter;
   A.coef_scale = P->d.coef_scale;

@@ -933,6 +933,9 @@ constexpr int CC_RED = 4;  // values reduced at once
 struct CcSolveArgs {
   CcArgs cc;
   float* x;        // solution, mean removed
+  float* x_raw;    // what the launched CG leaves in its vectors: x before that,
+  float* rhs;      // b without its mean (may be null),
+  float* res[2];   // and the last two residuals, in turn
   float tol;
   int max_iter;
   float coef_scale;
@@ -1062,6 +1065,21 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
     const unsigned m = in >> (4 * u + 2 * c);
     return f2_make(m & 1u ? x : 0.f, m & 2u ? y : 0.f);
   };
+  // a vector of the top level's cells plus a constant, to global memory
+  auto store = [&](float* g, unsigned v, float shift) {
+    float* out = g + (size_t)cy.lo * L.n1 * L.n2;
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      if (!mine || !cy.on(u)) continue;
+      int row, h;
+      cy.locate(L, u, row, h);
+      const f2 e0 = cy.vec(v, cy.odd(u), u), e1 = cy.vec(v, 1 - cy.odd(u), u);
+      const float w[4] = {f2_x(e0), f2_x(e1), f2_y(e0), f2_y(e1)};
+#pragma unroll
+      for (int d = 0; d < 4; ++d)
+        if (4 * h + d < L.n2) out[row * L.n2 + 4 * h + d] = w[d] + shift;
+    }
+  };
   auto amax = [](float x, float m) { return fmaxf(m, isfinite(x) ? fabsf(x) : INFINITY); };
   reduce(k1, sum, red);
   const double n = (double)A.n_total;
@@ -1080,11 +1098,12 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
         cc_sts2(cy.vec_at(Xv, c, u), f2_bcast(0.f));
       }
   }
+  if (A.rhs) store(A.rhs, Rv[0], 0.f);
   red[0] = (double)m;
   reduce(k1, mx, red);
   const double bnorm = red[0];
   double rel = 1.0, rz = 0.0, sum_r_old = 0.0;
-  int it = 0, status = ST_RUNNING;
+  int it = 0, updates = 0, status = ST_RUNNING;
   bool go = A.max_iter > 0;
   if (!(bnorm > 0.0) || isinf(bnorm)) {
     status = bnorm == 0.0 ? ST_ZERO_RHS : ST_NONFINITE;
@@ -1196,6 +1215,7 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
           cc_sts2(cy.vec_at(Rv[cur ^ 1], c, u), rn);
         }
       cur ^= 1;
+      ++updates;
     }
     red[0] = cy.fail ? (double)INFINITY : (double)m;  // a wait that ran out ends the iteration everywhere
     reduce(k1, mx, red);
@@ -1213,6 +1233,10 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
     }
   }
 
+  store(A.res[updates & 1], Rv[cur], 0.f);
+  if (updates > 0 && updates == it) store(A.res[(updates & 1) ^ 1], Rv[cur ^ 1], 0.f);
+  store(A.x_raw, Xv, 0.f);
+
   // ---- x with its mean removed
   red[0] = 0.0;
 #pragma unroll
@@ -1224,19 +1248,7 @@ __global__ void __launch_bounds__(CC_NT, 1) k_solve(const __grid_constant__ CcSo
       red[0] += (double)f2_x(x) + (double)f2_y(x);
     }
   reduce(k1, sum, red);
-  const float cx = (float)(-(red[0] / n));
-  float* out = A.x + (size_t)cy.lo * L.n1 * L.n2;
-#pragma unroll
-  for (int u = 0; u < NQ; ++u) {
-    if (!mine || !cy.on(u)) continue;
-    int row, h;
-    cy.locate(L, u, row, h);
-    const f2 x0 = cy.vec(Xv, cy.odd(u), u), x1 = cy.vec(Xv, 1 - cy.odd(u), u);
-    const float v[4] = {f2_x(x0), f2_x(x1), f2_y(x0), f2_y(x1)};
-#pragma unroll
-    for (int d = 0; d < 4; ++d)
-      if (4 * h + d < L.n2) out[row * L.n2 + 4 * h + d] = v[d] + cx;
-  }
+  store(A.x, Xv, (float)(-(red[0] / n)));
   if (cy.fail)
     asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(cc_map(smem_u32(&s_fail), L.c0)), "r"(1) : "memory");
   if (a.C > 1) cc_sync();  // no CTA leaves while another may still write to it

@@ -138,6 +138,31 @@ def test_one_launch_solve_matches_launched_cg(res, precision, stencil, tol):
     assert off(x1, x2) < 10 * tol
 
 
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+@pytest.mark.parametrize("max_iter", [0, 1, 2, 3])
+@pytest.mark.parametrize("res", [(16, 16, 16), (13, 11, 9), (32, 32, 32)])
+def test_one_launch_solve_leaves_the_vectors_of_the_launched_cg(res, max_iter, precision):
+    """x, rhs and the last two residuals, as the launched CG leaves them, from
+    vectors that hold something else before.  The iterates of the two part by
+    rounding: 1e-4 of the maximum (of b for the residuals), 1e-2 where the
+    preconditioner keeps 16 bits."""
+    bx, by, bz, b, _ = scenes.solve_problem(res, seed=37)
+    g = MGPCG(res, DEV, pre=2, post=2, precision=precision)
+    g.build_hierarchy(dev(bx), dev(by), dev(bz))
+    left = []
+    for verbose in (False, True):
+        for a in (g.x, g.rhs, g.res_v, g.r_prev):
+            a.fill_(7.0)
+        out = DeviceArray.zeros(res, device=DEV)
+        g.solve(dev(b), out, tol=1e-30, max_iter=max_iter, verbose=verbose)
+        left.append([a.numpy().astype(np.float64) for a in (g.x, g.rhs, g.res_v, g.r_prev, out)])
+    for k, (a, c) in enumerate(zip(*left)):
+        scale = np.abs(c if k in (0, 4) else left[1][1]).max()
+        assert np.abs(a - c).max() <= (1e-4 if precision == "fp32" else 1e-2) * scale, k
+    x, out = left[0][0], left[0][4]
+    assert np.abs(x - x.mean() - out).max() <= 1e-6 * max(np.abs(x).max(), 1e-30)
+
+
 @pytest.mark.parametrize("res", [(16, 16, 16), (32, 32, 32), (13, 11, 9)])
 def test_one_launch_solve_stops_like_the_launched_cg(res):
     bx, by, bz, b, _ = scenes.solve_problem(res, seed=35)
