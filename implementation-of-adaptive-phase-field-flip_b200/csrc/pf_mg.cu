@@ -2760,15 +2760,23 @@ template <class T> int enqueue_whole(pf_mg_plan* P, const float* b, float* x, fl
   return PF_OK;
 }
 
-// Iterations one launch may run: an iteration takes 15 to 60 us, so a launch ends
-// within 0.1 s.  Longer solves, and verbose ones (a line per iteration), launch
-// every iteration.
-constexpr int kWholeMaxIter = 1000;
+// Iterations one launch may run, so that it ends within 0.25 s: at most 25 us an
+// iteration outside its half-sweeps, which take up to 0.75 us (1.5 in FP64) each.
+// At 32^3 with 3 + 3 sweeps that is 5800 iterations, with a coarsest level swept 60
+// times over 1000, swept 2000 times 80.  Longer solves, and verbose ones (a line
+// per iteration), launch every iteration.
+int whole_max_iter(const pf_mg_plan* P) {
+  const CcArgs& a = P->cc;
+  const bool swept = a.nb == 0;
+  double half_sweeps = 2.0 * ((double)P->d.pre + P->d.post) * (swept ? a.nl - 1 : a.nl);
+  if (swept) half_sweeps += 2.0 * (double)P->d.coarsest * (mixed(P) ? 2.0 : 1.0);
+  return (int)(0.25e6 / (25.0 + 0.75 * half_sweeps));
+}
 
 template <class T>
 int solve_impl(pf_mg_plan* P, const float* b, float* x, float tol, int max_iter, int use_graphs, int verbose,
                int* iters_out, double* rel_out, cudaStream_t s) {
-  const bool whole = P->whole && !verbose && max_iter <= kWholeMaxIter;
+  const bool whole = P->whole && !verbose && max_iter <= whole_max_iter(P);
   if (whole) {
     PF_TRY(enqueue_whole<T>(P, b, x, tol, max_iter, s));
   } else {
@@ -3204,16 +3212,23 @@ int pf_mg_plan_create(const pf_mg_desc* desc, pf_mg_plan** out) {
   // k_coarse where its cluster can be resident; the dense operator needs its buffer
   P->lb = select_coarse(desc, &P->cc, &P->cc_nq, &P->cc_smem, &P->dense_l0);
   P->coarse = P->lb >= 0 && (P->cc.nb == 0 || (desc->bottom_op && (reinterpret_cast<uintptr_t>(desc->bottom_op) & 7u) == 0));
-  if (P->coarse && P->cc.C > 8) {
+  auto resident = [&](bool solve, size_t smem) {
+    if (P->cc.C <= 8) return true;
     cudaLaunchAttribute attr[2];
-    const cudaLaunchConfig_t cfg = coarse_config(P->cc.C, P->cc_smem, nullptr, attr);
-    void* k = desc->precision == PF_PREC_FP16   ? coarse_kernel<__half>(P->cc_nq)
-              : desc->precision == PF_PREC_BF16 ? coarse_kernel<__nv_bfloat16>(P->cc_nq)
-                                                : coarse_kernel<float>(P->cc_nq);
+    const cudaLaunchConfig_t cfg = coarse_config(P->cc.C, smem, nullptr, attr);
+    auto kernel = [&](auto t) {
+      using T = decltype(t);
+      return solve ? solve_kernel<T>(P->cc_nq) : coarse_kernel<T>(P->cc_nq);
+    };
+    void* k = desc->precision == PF_PREC_FP16   ? kernel(__half())
+              : desc->precision == PF_PREC_BF16 ? kernel(__nv_bfloat16())
+                                                : kernel(0.f);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) P->coarse = false;
+    const bool ok = cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= 1;
     cudaGetLastError();
-  }
+    return ok;
+  };
+  P->coarse = P->coarse && resident(false, P->cc_smem);
   if (P->coarse && P->lb == 0) {
     // the CG vectors behind k_coarse's shared memory
     const CcLevel& L = P->cc.L[0];
@@ -3229,7 +3244,7 @@ int pf_mg_plan_create(const pf_mg_desc* desc, pf_mg_plan** out) {
     P->cs.oR2 = take(v);
     P->cs.oX = take(v);
     P->cs_smem = off * sizeof(float);
-    P->whole = P->cs_smem <= (size_t)kCcSmemMax;
+    P->whole = P->cs_smem <= (size_t)kCcSmemMax && resident(true, P->cs_smem);
   }
   if (!P->coarse) {
     const BottomSel sel = select_bottom(desc);

@@ -98,9 +98,10 @@ class MGPCG:
     After a solve ``x`` is the solution before its mean is removed, ``rhs`` the
     right-hand side without its mean, and ``res_v`` (an even number of updates) or
     ``r_prev`` (odd) the last residual, the other one the residual before.  A solve
-    of up to about 40^3 cells that is not verbose runs in one launch, whatever
-    ``use_graphs`` says: ``z``, ``q``, ``Ap`` and the levels' ``p`` then keep what
-    they held."""
+    of up to about 40^3 cells runs in one launch, whatever ``use_graphs`` says,
+    unless it is verbose, max_iter times its sweeps could take above 0.25 s, or (in
+    16-bit hierarchies) the dense operator of the smallest levels fills the shared
+    memory: ``z``, ``q``, ``Ap`` and the levels' ``p`` then keep what they held."""
 
     def __init__(self, res, device="cuda:0", *, omega=6.0 / 7.0, pre=2, post=2, coarsest=60, min_dim=4,
                  precision="fp32", stencil="flux", coef_scale=None, use_graphs=True):

@@ -16,6 +16,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
+from pfflip import _native as N
 from pfflip import scenes
 from pfflip._arrays import DeviceArray
 from pfflip.poisson import MGPCG
@@ -112,13 +113,15 @@ def test_16bit_swept_coarsest_level_is_swept_in_binary64(res, first, precision, 
     assert not (np.abs(z[""] - z["cta"]) > step * np.abs(z["cta"])).any()
 
 
-def solves(g, res, b, tol, max_iter):
+def solves(g, res, b, tol, max_iter, one=True):
     """(iterations, residual, x) of the one-launch solve and of the launched CG
-    (verbose solves take that one)."""
+    (verbose solves take that one; with `one` False both do)."""
     out = []
     for verbose in (False, True):
-        x = DeviceArray.zeros(res, device=DEV)
-        it, rel = g.solve(dev(b), x, tol=tol, max_iter=max_iter, verbose=verbose)
+        x, rhs = DeviceArray.zeros(res, device=DEV), dev(b)
+        before = N.launch_count()
+        it, rel = g.solve(rhs, x, tol=tol, max_iter=max_iter, verbose=verbose)
+        assert (N.launch_count() - before == 1) == (one and not verbose)
         out.append((it, rel, x.numpy().astype(np.float64)))
     return out
 
@@ -132,10 +135,27 @@ def test_one_launch_solve_matches_launched_cg(res, precision, stencil, tol):
     bx, by, bz, b, _ = scenes.solve_problem(res, seed=34)
     g = MGPCG(res, DEV, pre=3, post=3, precision=precision, stencil=stencil)
     g.build_hierarchy(dev(bx), dev(by), dev(bz))
-    (i1, r1, x1), (i2, r2, x2) = solves(g, res, b, tol, 200)
+    # the binary64 operator of 8^3 cells leaves no room for the CG vectors
+    one = precision == "fp32" or res not in ((16, 16, 16), (32, 32, 32))
+    (i1, r1, x1), (i2, r2, x2) = solves(g, res, b, tol, 200, one)
     assert r1 < tol and r2 < tol and abs(i1 - i2) <= 1, (i1, r1, i2, r2)
     assert abs(x1.mean()) < 1e-6 * np.abs(x1).max()
     assert off(x1, x2) < 10 * tol
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+@pytest.mark.parametrize("coarsest,max_iter,one", [(60, 1000, True), (60, 4000, False), (2000, 200, False), (2000, 10, True)])
+def test_one_launch_is_bounded_in_time(coarsest, max_iter, one, precision):
+    """A launch that could take above 0.25 s is left to the launched CG."""
+    res = (13, 11, 9)  # one level, swept
+    bx, by, bz, b, _ = scenes.solve_problem(res, seed=38)
+    g = MGPCG(res, DEV, coarsest=coarsest, precision=precision)
+    g.build_hierarchy(dev(bx), dev(by), dev(bz))
+    x, rhs = DeviceArray.zeros(res, device=DEV), dev(b)
+    before = N.launch_count()
+    it, rel = g.solve(rhs, x, tol=1e-5, max_iter=max_iter)
+    assert (N.launch_count() - before == 1) == one
+    assert rel < 1e-5
 
 
 @pytest.mark.parametrize("precision", ["fp32", "fp16"])
