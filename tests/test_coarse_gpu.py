@@ -42,25 +42,29 @@ def off(a, b):
     return np.abs(a - b).max() / np.abs(b).max()
 
 
-SHAPES = [
-    (4, 4, 4),  # a single level on one CTA
-    (13, 11, 9),  # a single odd level, swept; rows of 9
-    (21, 23, 27),  # a single odd level in slabs
-    (24, 24, 24),  # slabs, one CTA, dense 6^3
-    (20, 20, 22),  # 10 x 10 x 11 swept
-    (30, 22, 18),  # rows of 18 and 9
-    (38, 44, 38),  # three quads a thread, coarsest 19 x 22 x 19 in slabs
-    (48, 32, 40),  # two levels on the same CTAs
-    (16, 64, 24),  # one plane per slab
-    (62, 30, 34),  # a launched level above 31 x 15 x 17
-]
+# extents: (first level, swept levels on a cluster, dense operator)
+SHAPES = {
+    (4, 4, 4): (0, 0, 0),  # a single level on one CTA
+    (13, 11, 9): (0, 0, 0),  # a single odd level, swept; rows of 9
+    (21, 23, 27): (0, 1, 0),  # a single odd level in slabs
+    (24, 24, 24): (0, 2, 1),  # slabs, one CTA, dense 6^3
+    (20, 20, 22): (0, 2, 0),  # 10 x 10 x 11 swept
+    (30, 22, 18): (0, 2, 0),  # rows of 18 and 9
+    (38, 44, 38): (0, 2, 0),  # three quads a thread, coarsest 19 x 22 x 19 in slabs
+    (48, 32, 40): (0, 3, 1),  # two levels on the same CTAs
+    (16, 64, 24): (0, 2, 1),  # one plane per slab
+    (62, 30, 34): (0, 2, 0),  # four planes a slab, three quads a thread
+    (64, 48, 48): (1, 2, 1),  # a launched level above
+    (62, 60, 68): (1, 1, 0),  # a launched level above a swept 31 x 30 x 34
+}
 
 
 @pytest.mark.parametrize("stencil", ["flux", "reference"])
 @pytest.mark.parametrize("res", SHAPES)
 def test_coarse_vcycle_matches_oracle(res, stencil):
     bx, by, bz, b, _ = scenes.solve_problem(res, seed=31)
-    _, z = vcycle(res, bx, by, bz, b, pre=3, post=3, stencil=stencil)
+    g, z = vcycle(res, bx, by, bz, b, pre=3, post=3, stencil=stencil)
+    assert g.bottom_info() == SHAPES[res]
     o = O.OracleMGPCG(res, pre=3, post=3, stencil=stencil)
     o.build_hierarchy(bx, by, bz)
     assert off(z, o.precondition(b).astype(np.float64)) < 2e-4
@@ -181,6 +185,40 @@ def test_one_launch_solve_leaves_the_vectors_of_the_launched_cg(res, max_iter, p
         assert np.abs(a - c).max() <= (1e-4 if precision == "fp32" else 1e-2) * scale, k
     x, out = left[0][0], left[0][4]
     assert np.abs(x - x.mean() - out).max() <= 1e-6 * max(np.abs(x).max(), 1e-30)
+
+
+@pytest.mark.parametrize("precision,stencil", [("fp32", "flux"), ("fp32", "reference"), ("fp16", "flux"), ("bf16", "flux")])
+@pytest.mark.parametrize("res", [(13, 11, 9), (21, 23, 27), (24, 24, 24), (30, 22, 18), (40, 40, 40)])
+def test_one_launch_solve_matches_binary64(res, precision, stencil):
+    """The one-launch solve against the CPU oracle in binary64 at 1e-12: within
+    10 tol of the maximum, as the other solves."""
+    tol = 1e-6 if stencil == "flux" else 1e-4
+    bx, by, bz, b, _ = scenes.solve_problem(res, seed=39)
+    g = MGPCG(res, DEV, pre=3, post=3, precision=precision, stencil=stencil)
+    g.build_hierarchy(dev(bx), dev(by), dev(bz))
+    x, rhs = DeviceArray.zeros(res, device=DEV), dev(b)
+    before = N.launch_count()
+    it, rel = g.solve(rhs, x, tol=tol, max_iter=300)
+    assert N.launch_count() - before == 1 and rel < tol, (it, rel)
+    x64, _, _ = O.fp64_reference_solve(bx, by, bz, b.astype(np.float64), tol=1e-12)
+    assert off(x.numpy().astype(np.float64), x64) < 10 * tol
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16"])
+def test_launched_graph_and_eager_solves_are_bitwise_equal(precision):
+    """Above the sizes that run in one launch, where use_graphs matters."""
+    res = (64, 48, 48)
+    bx, by, bz, b, _ = scenes.solve_problem(res, seed=40)
+    outs = []
+    for graphs in (True, False, True):
+        g = MGPCG(res, DEV, pre=3, post=3, use_graphs=graphs, precision=precision)
+        g.build_hierarchy(dev(bx), dev(by), dev(bz))
+        x, rhs = DeviceArray.zeros(res, device=DEV), dev(b)
+        before = N.launch_count()
+        outs.append((g.solve(rhs, x, tol=1e-6, max_iter=100), x.numpy()))
+        assert N.launch_count() - before > 10
+    for o in outs[1:]:
+        assert o[0] == outs[0][0] and np.array_equal(o[1], outs[0][1])
 
 
 @pytest.mark.parametrize("res", [(16, 16, 16), (32, 32, 32), (13, 11, 9)])
