@@ -834,7 +834,7 @@ __global__ void k_residual_restrict(int n0, int n1, int n2, const T* __restrict_
 // half-sweeps separated by barriers.  Replaces ~7 launches per level.  The
 // coarsest level runs in AccT (float reproduces the reference; double is the
 // FP64 coarsest solve of the 16-bit hierarchy), by one warp when it has at most
-// 256 cells.
+// 64 cells.
 constexpr int kBottomMaxCells = 4096;
 constexpr int BT_NT = 1024;
 

@@ -32,7 +32,7 @@
 // Measured on a B200, per V-cycle inside a solve, against one CTA holding the
 // levels of up to 4096 cells (and an 8-CTA cluster where every extent is a
 // multiple of 16) with launched sweeps above: 16^3 40 -> 18 us, 32^3 and below
-// 53 -> 35 us, 24^3 (coarsest 6^3) 128 + 6 sweeps of 5 us -> 21 us, 30x22x18
+// 52 -> 33 us, 24^3 (coarsest 6^3) 128 + 6 sweeps of 5 us -> 21 us, 30x22x18
 // (coarsest 15x11x9 swept) 167 + 6 of 8 us -> 41 us, 31^3 swept 60 times
 // 600 -> 62 us.  A half-sweep takes 0.5 us on one CTA (its shared-memory
 // wavefronts are 0.2 us of that) and 0.7 us with the exchange.

@@ -172,10 +172,10 @@ class MGPCG:
 
     def bottom_info(self):
         """``(first_level, cluster_levels, dense)`` of the kernel that runs the
-        coarse end of the V-cycle: cluster_levels > 0 for the CTA-cluster
-        kernel, 0 for the single-CTA one; dense = 1 when the levels below the
-        cluster's slabs run as a dense operator (diagnostics; no reference
-        counterpart)."""
+        coarse end of the V-cycle: cluster_levels is the number of levels it
+        sweeps on a cluster of CTAs, 0 where one CTA runs them; dense = 1 when
+        the levels below those are applied as a dense operator (diagnostics; no
+        reference counterpart)."""
         first, nd, dense = C.c_int32(0), C.c_int32(0), C.c_int32(0)
         N.call("pf_mg_bottom_info", self._plan, C.byref(first), C.byref(nd), C.byref(dense))
         return int(first.value), int(nd.value), int(dense.value)
